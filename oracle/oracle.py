@@ -25,6 +25,8 @@ REF_VAMANA = os.path.join(HERE, "_ref", "Vamana")
 # reads them there); NBPG_REF_ROOT overrides the location, and a machine without them builds the
 # restatement only
 REF_ROOT = os.environ.get("NBPG_REF_ROOT", "/root/reference")
+if not os.path.isdir(os.path.join(REF_ROOT, "algorithms")):
+    REF_ROOT = ""  # an empty checkout folder counts as absent
 
 DTYPES = {"u8": 0, "i8": 1, "u4": 2, "i4": 3, "f32": 4}
 METRICS = {"l2": 0, "ip": 1}
