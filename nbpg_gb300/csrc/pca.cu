@@ -23,10 +23,9 @@
 
 namespace nbpg {
 
-constexpr int PCA_PTS = 32;    // points per CTA
-constexpr int PCA_OUTS = 64;   // outputs per CTA
-constexpr int PCA_THREADS = 256;
-constexpr uint32_t PCA_MAX_DIN = 576;  // shared memory: d_in x 384 B + 8 KB
+constexpr uint32_t PCA_MAX_DIN = 576;
+constexpr int PCA_THREADS = 256;  // 8 (outputs) x 32 (points)
+constexpr int PCA_KC = 32;        // input elements staged per round
 
 enum PcaIn : int { PIN_F32 = 0, PIN_U8 = 1, PIN_I8 = 2 };
 
@@ -38,76 +37,211 @@ __device__ __forceinline__ float load_in(const void *x, uint64_t i)
     else return float(static_cast<const int8_t *>(x)[i]);
 }
 
+// int((v + 1) * 0.5 * 255) as matrix.h:112 evaluates it (float add, double products, truncation),
+// clamped to [0, 255], without the scarce FP64 units.  s = v + 1 has 24 significant bits, so the
+// double product is the exact s * 127.5; p = s * 127.5 rounded to float and its exact error e from
+// an FMA hold the same value, and p's truncation is off only where p was rounded up onto an integer.
 __device__ __forceinline__ int quant_code(float v)
 {
-    const double t = __dmul_rn(__dmul_rn(double(__fadd_rn(v, 1.0f)), 0.5), 255.0);
-    return __double2int_rz(t);  // saturates; NaN gives 0, which clamps like the low end
+    const float s = __fadd_rn(v, 1.0f);
+    const float p = __fmul_rn(s, 127.5f);
+    const float e = __fmaf_rn(s, 127.5f, -p);
+    int t = __float2int_rz(p);  // saturates; NaN gives 0
+    if (float(t) == p && e < 0.0f) --t;
+    return min(max(t, 0), 255);
 }
 
-// grid (ceil(n / 32), ceil(d_out / 64)); out_kind: 0 f32, 1 u8, 2 i8, 3 u4, 4 i4
-template <int IN>
-__global__ void __launch_bounds__(PCA_THREADS) pca_kernel(const void *x, uint64_t n, uint32_t d_in, const float *mat,
-                                                         const float *bias, uint32_t d_out, uint32_t out_kind,
-                                                         void *out)
+__device__ __forceinline__ uint64_t pair2(float lo, float hi)
 {
-    extern __shared__ float sm[];
-    float *mT = sm;                                   // [d_in][64]
-    float *xs = mT + size_t(d_in) * PCA_OUTS;         // [32][d_in]
-    float *vals = xs + size_t(PCA_PTS) * d_in;        // [32][64]
-    const int tid = threadIdx.x;
-    const uint32_t j0 = blockIdx.y * PCA_OUTS;
-    const uint64_t p0 = uint64_t(blockIdx.x) * PCA_PTS;
-    for (uint32_t e = tid; e < d_in * PCA_OUTS; e += PCA_THREADS) {
-        const uint32_t c = e % PCA_OUTS, i = e / PCA_OUTS;
-        mT[e] = j0 + c < d_out ? mat[size_t(j0 + c) * d_in + i] : 0.0f;
-    }
-    for (uint32_t e = tid; e < PCA_PTS * d_in; e += PCA_THREADS) {
-        const uint32_t pl = e / d_in, i = e % d_in;
-        xs[e] = p0 + pl < n ? load_in<IN>(x, (p0 + pl) * d_in + i) : 0.0f;
-    }
-    __syncthreads();
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+// acc + a * b on two values at once, the product rounded before the sum.  The sum is written as
+// product * one + acc, with `one` = (1, 1) from a kernel argument: the same rounding as an add, and
+// nothing an optimiser may contract with the product (mul.f32x2 followed by add.f32x2 came out as
+// one FMA, which rounds once and moved codes).
+__device__ __forceinline__ void mul_add2(uint64_t &acc, uint64_t a, uint64_t b, uint64_t one)
+{
+    uint64_t t;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(t) : "l"(a), "l"(b));
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(t), "l"(one));
+}
 
-    const int g = tid / PCA_OUTS, c = tid % PCA_OUTS;  // 4 groups of 8 points
-    float acc[8];
+// Column of output `o` (0 .. OPT - 1) of a thread with output lane tx: four neighbours in the first
+// 32 columns, the rest beside each other from column 32 on, so that a warp's 8 output lanes read
+// neighbouring vectors of shared memory and a 4-bit pair stays within one thread.
+template <int OPT>
+__device__ __forceinline__ uint32_t pca_col(uint32_t tx, int o)
+{
+    return o < 4 ? tx * 4 + o : 32 + tx * (OPT - 4) + (o - 4);
+}
+
+// One CTA: 32 * PPT points x 8 * OPT outputs; a thread owns PPT points x OPT outputs in registers
+// and walks the input elements in index order, so every output keeps the reference's summation order.
+// What bounds it: one multiply and one add per input element and output (two instructions, no FMA):
+// 16.4 G lane operations for 1M x 128 -> 64, 0.42 ms on 152 SMs x 128 lanes at 2 GHz, against 0.08 ms
+// of HBM traffic; it measures 0.67 ms (1.70 ms with one output x 8 points per thread, a whole d_in of
+// both operands in shared memory and double-precision quantisation).  Hence a register tile (16 shared-memory values feed 64 multiply-adds) and
+// two-wide mul / add, which leave issue slots for the loads.  xs[i][p] is stored with its point
+// index XORed by 4 * ((i / 4) % 8): the transposing stores and the 16-byte reads are both free of
+// bank conflicts.
+// out_kind: 0 f32, 1 u8, 2 i8, 3 u4, 4 i4; vec: rows of x are 16-byte (f32) or 4-byte (codes) aligned
+// and d_in is a multiple of 4; wide: d_out is a multiple of 4 and out 16-byte aligned, so four outputs
+// of a thread are one store.
+template <int IN, int PPT, int OPT>
+__global__ void __launch_bounds__(PCA_THREADS, 2) pca_kernel(const void *x, uint64_t n, uint32_t d_in, const float *mat,
+                                                            const float *bias, uint32_t d_out, uint32_t out_kind,
+                                                            uint32_t vec, uint32_t wide, float one, void *out)
+{
+    constexpr int P = 32 * PPT, O = 8 * OPT;
+    __shared__ __align__(16) float xs[PCA_KC * P];
+    __shared__ __align__(16) float ms[PCA_KC * O];
+    const uint32_t tid = threadIdx.x, tx = tid & 7, ty = tid >> 3;
+    const uint32_t j0 = blockIdx.y * O;
+    const uint64_t p0 = uint64_t(blockIdx.x) * P;
+    const uint64_t one2 = pair2(one, one);
+    uint64_t acc[PPT][OPT / 2];
 #pragma unroll
-    for (int q = 0; q < 8; ++q) acc[q] = 0.0f;
-    for (uint32_t i = 0; i < d_in; ++i) {
-        const float m = mT[i * PCA_OUTS + c];
+    for (int q = 0; q < PPT; ++q)
 #pragma unroll
-        for (int q = 0; q < 8; ++q) acc[q] = __fadd_rn(acc[q], __fmul_rn(m, xs[(g * 8 + q) * d_in + i]));
-    }
-    const uint32_t j = j0 + c;
-    const float b = j < d_out ? bias[j] : 0.0f;
+        for (int o = 0; o < OPT / 2; ++o) acc[q][o] = 0;
+
+    for (uint32_t i0 = 0; i0 < d_in; i0 += PCA_KC) {
+        const uint32_t kc = min(uint32_t(PCA_KC), d_in - i0);
+        if (i0) __syncthreads();
+        if (vec) {
+            // 8 threads per row, 4 elements each
+            float4 v[PPT];
+            const uint32_t i = i0 + tx * 4;
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {
-        const float v = __fadd_rn(b, acc[q]);  // bias - (-dot)
-        const uint64_t p = p0 + g * 8 + q;
-        if (out_kind == 0) {
-            if (p < n && j < d_out) static_cast<float *>(out)[p * d_out + j] = v;
+            for (int r = 0; r < PPT; ++r) {
+                const uint64_t p = p0 + r * 32 + ty;
+                v[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (p < n && i < d_in) {
+                    if constexpr (IN == PIN_F32) {
+                        v[r] = __ldcs(reinterpret_cast<const float4 *>(static_cast<const float *>(x) + p * d_in + i));
+                    } else if constexpr (IN == PIN_U8) {
+                        const uchar4 c = *reinterpret_cast<const uchar4 *>(static_cast<const uint8_t *>(x) + p * d_in + i);
+                        v[r] = make_float4(c.x, c.y, c.z, c.w);
+                    } else {
+                        const char4 c = *reinterpret_cast<const char4 *>(static_cast<const int8_t *>(x) + p * d_in + i);
+                        v[r] = make_float4(float(int8_t(c.x)), float(int8_t(c.y)), float(int8_t(c.z)), float(int8_t(c.w)));
+                    }
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < PPT; ++r) {
+                float *d = xs + tx * 4 * P + ((r * 32 + ty) ^ (4 * tx));
+                d[0] = v[r].x;
+                d[P] = v[r].y;
+                d[2 * P] = v[r].z;
+                d[3 * P] = v[r].w;
+            }
         } else {
-            vals[(g * 8 + q) * PCA_OUTS + c] = v;
+            for (uint32_t e = tid; e < P * PCA_KC; e += PCA_THREADS) {
+                const uint32_t pl = e / PCA_KC, i = e % PCA_KC;
+                const uint64_t p = p0 + pl;
+                xs[i * P + (pl ^ (4 * ((i >> 2) & 7)))] = p < n && i < kc ? load_in<IN>(x, p * d_in + i0 + i) : 0.0f;
+            }
+        }
+        for (uint32_t e = tid; e < O * PCA_KC; e += PCA_THREADS) {
+            const uint32_t i = e % PCA_KC, j = e / PCA_KC;
+            ms[i * O + j] = i < kc && j0 + j < d_out ? __ldg(mat + size_t(j0 + j) * d_in + i0 + i) : 0.0f;
+        }
+        __syncthreads();
+        for (uint32_t i = 0; i < kc; ++i) {
+            float xv[PPT];
+            const float *xr = xs + i * P;
+            const uint32_t sw = 4 * ((i >> 2) & 7);
+            if constexpr (PPT >= 4) {
+#pragma unroll
+                for (int q = 0; q < PPT; q += 4) {
+                    const float4 t = *reinterpret_cast<const float4 *>(xr + ((ty * PPT + q) ^ sw));
+                    xv[q] = t.x;
+                    xv[q + 1] = t.y;
+                    xv[q + 2] = t.z;
+                    xv[q + 3] = t.w;
+                }
+            } else {
+                const float2 t = *reinterpret_cast<const float2 *>(xr + ((ty * PPT) ^ sw));
+                xv[0] = t.x;
+                xv[1] = t.y;
+            }
+            uint64_t mv[OPT / 2];
+            const float *mr = ms + i * O;
+            {
+                const ulonglong2 t = *reinterpret_cast<const ulonglong2 *>(mr + tx * 4);
+                mv[0] = t.x;
+                mv[1] = t.y;
+            }
+            if constexpr (OPT == 6) mv[2] = *reinterpret_cast<const uint64_t *>(mr + 32 + tx * 2);
+            if constexpr (OPT == 8) {
+                const ulonglong2 t = *reinterpret_cast<const ulonglong2 *>(mr + 32 + tx * 4);
+                mv[2] = t.x;
+                mv[3] = t.y;
+            }
+#pragma unroll
+            for (int q = 0; q < PPT; ++q) {
+                const uint64_t xx = pair2(xv[q], xv[q]);
+#pragma unroll
+                for (int o = 0; o < OPT / 2; ++o) mul_add2(acc[q][o], mv[o], xx, one2);
+            }
         }
     }
-    if (out_kind == 0) return;
-    __syncthreads();
+
     const uint32_t chunk = out_kind >= 3 ? 2 : 1;
     const int delta = (out_kind == 2 || out_kind == 4) ? 128 : 0;
-    const int offset = 8 - 8 / int(chunk), mask = (1 << (8 / chunk)) - 1;
-    const uint32_t out_dims = d_out / chunk, bpp = PCA_OUTS / chunk;
-    for (uint32_t e = tid; e < PCA_PTS * bpp; e += PCA_THREADS) {
-        const uint32_t pl = e / bpp, bi = e % bpp;
-        const uint32_t ob = j0 / chunk + bi;
-        const uint64_t p = p0 + pl;
-        if (p >= n || ob >= out_dims) continue;
-        uint32_t res = 0;
-        for (uint32_t jj = 0; jj < chunk; ++jj) {
-            const float v = vals[pl * PCA_OUTS + (bi + 1) * chunk - 1 - jj];
-            res = (res << (8 / chunk)) & 0xFFu;
-            int ti = quant_code(v);
-            ti = (min(max(ti, 0), 255) - delta) >> offset;
-            res = (res + uint32_t(ti & mask)) & 0xFFu;
+    const uint32_t width = d_out / chunk;
+#pragma unroll
+    for (int q = 0; q < PPT; ++q) {
+        const uint64_t p = p0 + ty * PPT + q;
+        if (p >= n) break;
+#pragma unroll
+        for (int o = 0; o < OPT; o += 4) {
+            constexpr int kMost = 4;
+            const int cnt = OPT - o < kMost ? OPT - o : kMost;  // 4, or the 2 past column 32 of OPT = 6
+            const uint32_t j = j0 + pca_col<OPT>(tx, o);
+            float v[kMost];
+#pragma unroll
+            for (int c = 0; c < kMost; c += 2)
+                if (c < cnt) asm("mov.b64 {%0, %1}, %2;" : "=f"(v[c]), "=f"(v[c + 1]) : "l"(acc[q][(o + c) / 2]));
+#pragma unroll
+            for (int c = 0; c < kMost; ++c)
+                if (c < cnt) v[c] = __fadd_rn(j + c < d_out ? __ldg(bias + j + c) : 0.0f, v[c]);  // bias - (-dot)
+            if (out_kind == 0) {
+                float *d = static_cast<float *>(out) + p * d_out + j;
+                if (wide && j + cnt <= d_out) {
+                    if (cnt == 4) __stcs(reinterpret_cast<float4 *>(d), make_float4(v[0], v[1], v[2], v[3]));
+                    else __stcs(reinterpret_cast<float2 *>(d), make_float2(v[0], v[1]));
+                } else {
+#pragma unroll
+                    for (int c = 0; c < kMost; ++c)
+                        if (c < cnt && j + c < d_out) d[c] = v[c];
+                }
+                continue;
+            }
+            uint32_t code[kMost] = {0, 0, 0, 0};
+#pragma unroll
+            for (int c = 0; c < kMost; ++c)
+                if (c < cnt) code[c] = uint32_t(quant_code(v[c]) - delta) & 0xFFu;
+            uint8_t *d = static_cast<uint8_t *>(out) + p * width + j / chunk;
+            if (chunk == 2) {  // high nibble = element 2i + 1 (j and d_out are even)
+                const uint32_t lo = (code[1] & 0xF0u) | (code[0] >> 4), hi = (code[3] & 0xF0u) | (code[2] >> 4);
+                if (wide && cnt == 4 && j + 4 <= d_out) {
+                    *reinterpret_cast<uint16_t *>(d) = uint16_t(lo | (hi << 8));
+                } else {
+                    if (j < d_out) d[0] = uint8_t(lo);
+                    if (cnt == 4 && j + 2 < d_out) d[1] = uint8_t(hi);
+                }
+            } else if (wide && cnt == 4 && j + 4 <= d_out) {
+                *reinterpret_cast<uint32_t *>(d) = code[0] | (code[1] << 8) | (code[2] << 16) | (code[3] << 24);
+            } else {
+#pragma unroll
+                for (int c = 0; c < kMost; ++c)
+                    if (c < cnt && j + c < d_out) d[c] = uint8_t(code[c]);
+            }
         }
-        static_cast<uint8_t *>(out)[p * out_dims + ob] = uint8_t(res);
     }
 }
 
@@ -135,11 +269,6 @@ __global__ void f32_to_u8_kernel(const float *rows, uint64_t count, uint8_t *out
     }
 }
 
-static size_t pca_smem(uint32_t d_in)
-{
-    return (size_t(d_in) * PCA_OUTS + size_t(PCA_PTS) * d_in + PCA_PTS * PCA_OUTS) * sizeof(float);
-}
-
 static uint32_t out_width(uint32_t out_dtype, uint32_t d_out)
 {
     return (out_dtype == NBPG_U4 || out_dtype == NBPG_I4) ? d_out / 2 : d_out;
@@ -156,31 +285,42 @@ static int out_kind_of(uint32_t out_dtype)
     }
 }
 
+template <int IN, int PPT>
+static void launch_pca_outs(uint32_t opt, dim3 grid, cudaStream_t st, const void *x, uint64_t n, uint32_t d_in,
+                            const float *mat, const float *bias, uint32_t d_out, uint32_t kind, uint32_t vec, uint32_t wide, void *out)
+{
+    if (opt == 4) pca_kernel<IN, PPT, 4><<<grid, PCA_THREADS, 0, st>>>(x, n, d_in, mat, bias, d_out, kind, vec, wide, 1.0f, out);
+    else if (opt == 6) pca_kernel<IN, PPT, 6><<<grid, PCA_THREADS, 0, st>>>(x, n, d_in, mat, bias, d_out, kind, vec, wide, 1.0f, out);
+    else pca_kernel<IN, PPT, 8><<<grid, PCA_THREADS, 0, st>>>(x, n, d_in, mat, bias, d_out, kind, vec, wide, 1.0f, out);
+}
+
+template <int IN>
+static void launch_pca_in(uint32_t ppt, uint32_t opt, dim3 grid, cudaStream_t st, const void *x, uint64_t n, uint32_t d_in,
+                          const float *mat, const float *bias, uint32_t d_out, uint32_t kind, uint32_t vec, uint32_t wide, void *out)
+{
+    if (ppt == 8) launch_pca_outs<IN, 8>(opt, grid, st, x, n, d_in, mat, bias, d_out, kind, vec, wide, out);
+    else launch_pca_outs<IN, 2>(opt, grid, st, x, n, d_in, mat, bias, d_out, kind, vec, wide, out);
+}
+
 static nbpg_status launch_pca(uint32_t in_dtype, const void *d_x, uint64_t n, uint32_t d_in, const float *d_mat,
                               const float *d_bias, uint32_t d_out, uint32_t out_dtype, void *d_out_rows,
                               cudaStream_t st)
 {
-    const size_t smem = pca_smem(d_in);
-    const dim3 grid(uint32_t((n + PCA_PTS - 1) / PCA_PTS), (d_out + PCA_OUTS - 1) / PCA_OUTS);
+    // columns per CTA: 32 or 48 where they cover d_out (no columns computed for padding), else 64
+    const uint32_t opt = d_out <= 32 ? 4 : d_out <= 48 ? 6 : 8;
+    // 256-point tiles once they fill every SM's two CTAs (2 x 152 x 256 = 78k points), else 64-point ones
+    const uint32_t ppt = n >= 80000 ? 8 : 2;
+    const uint32_t pts = 32 * ppt, outs = 8 * opt;
+    const dim3 grid(uint32_t((n + pts - 1) / pts), (d_out + outs - 1) / outs);
     const uint32_t kind = uint32_t(out_kind_of(out_dtype));
-    cudaError_t e;
+    const uint32_t vec = d_in % 4 == 0 && reinterpret_cast<uintptr_t>(d_x) % (in_dtype == NBPG_F32 ? 16 : 4) == 0;
+    const uint32_t wide = d_out % 4 == 0 && reinterpret_cast<uintptr_t>(d_out_rows) % 16 == 0;
     switch (in_dtype) {
-    case NBPG_F32:
-        e = cudaFuncSetAttribute(pca_kernel<PIN_F32>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-        if (e == cudaSuccess)
-            pca_kernel<PIN_F32><<<grid, PCA_THREADS, smem, st>>>(d_x, n, d_in, d_mat, d_bias, d_out, kind, d_out_rows);
-        break;
-    case NBPG_U8:
-        e = cudaFuncSetAttribute(pca_kernel<PIN_U8>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-        if (e == cudaSuccess)
-            pca_kernel<PIN_U8><<<grid, PCA_THREADS, smem, st>>>(d_x, n, d_in, d_mat, d_bias, d_out, kind, d_out_rows);
-        break;
-    default:
-        e = cudaFuncSetAttribute(pca_kernel<PIN_I8>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-        if (e == cudaSuccess)
-            pca_kernel<PIN_I8><<<grid, PCA_THREADS, smem, st>>>(d_x, n, d_in, d_mat, d_bias, d_out, kind, d_out_rows);
+    case NBPG_F32: launch_pca_in<PIN_F32>(ppt, opt, grid, st, d_x, n, d_in, d_mat, d_bias, d_out, kind, vec, wide, d_out_rows); break;
+    case NBPG_U8: launch_pca_in<PIN_U8>(ppt, opt, grid, st, d_x, n, d_in, d_mat, d_bias, d_out, kind, vec, wide, d_out_rows); break;
+    default: launch_pca_in<PIN_I8>(ppt, opt, grid, st, d_x, n, d_in, d_mat, d_bias, d_out, kind, vec, wide, d_out_rows);
     }
-    if (e == cudaSuccess) e = cudaGetLastError();
+    const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
         set_error(std::string("nbpg_pca_encode: ") + cudaGetErrorString(e));
         return NBPG_ERR_CUDA;

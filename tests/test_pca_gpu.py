@@ -144,3 +144,36 @@ def test_config3_pipeline(gpu_lib, oracle_lib, kind):
     rec_float = np.mean([len(set(a) & set(b)) / 10 for a, b in zip(res.ids[:, :10], exact)])
     ceiling = np.mean([len(set(a) & set(b)) / 10 for a, b in zip(code_gt, exact)])
     assert rec_float >= 0.9 * ceiling and ceiling > 0.1, (rec_float, ceiling)
+
+
+@pytest.mark.parametrize("n,d_in,d_out,kin,kout", [
+    (1, 4, 2, "f32", "u4"), (63, 33, 24, "f32", "f32"), (64, 31, 32, "u8", "i4"), (65, 32, 33, "f32", "u8"),
+    (255, 7, 47, "i8", "i8"), (1023, 36, 48, "f32", "u4"), (511, 100, 50, "u8", "u4"), (300, 64, 130, "f32", "f32"),
+    (79_999, 128, 64, "f32", "u4"), (80_000, 40, 64, "i8", "i4"), (80_257, 65, 46, "f32", "f32"),
+    (80_001, 44, 30, "u8", "u8"), (81_921, 28, 66, "f32", "i8")])
+def test_encode_tile_edges(gpu_lib, oracle_lib, n, d_in, d_out, kin, kout):
+    """Both point tiles (64 and 256 points, from 80,000 rows on), the three column tiles (32, 48 and
+    64 outputs), whole and ragged, rows that take the vector loads and rows that do not."""
+    from nbpg_gb300.pca import encode
+    r = np.random.default_rng(n + d_in)
+    if kin == "f32":
+        x, scale = r.normal(size=(n, d_in)).astype(np.float32), 0.5 / np.sqrt(d_in)
+    else:
+        lo, hi, t = (0, 256, np.uint8) if kin == "u8" else (-128, 128, np.int8)
+        x, scale = r.integers(lo, hi, (n, d_in)).astype(t), 0.5 / (128 * np.sqrt(d_in))
+    mat = (r.normal(size=(d_out, d_in)) * scale).astype(np.float32)
+    bias = (r.normal(size=d_out) * 0.2).astype(np.float32)
+    got, want = encode(x, mat, bias, kout), oracle_lib.pca_encode(x, mat, bias, kout)
+    assert np.array_equal(got.view(np.uint8), want.view(np.uint8))
+
+
+@pytest.mark.parametrize("kout", ["u8", "i8", "u4", "i4"])
+def test_encode_code_boundaries(gpu_lib, oracle_lib, kout):
+    """Values on, one float below and one float above every code boundary k / 127.5 - 1."""
+    from nbpg_gb300.pca import encode
+    edge = (np.arange(-3, 260, dtype=np.float64) / 127.5 - 1.0).astype(np.float32)
+    v = np.concatenate([edge, np.nextafter(edge, np.float32(-9)), np.nextafter(edge, np.float32(9)),
+                        np.float32([-0.0, 0.0, 1e-30, -1e-30, 1.0, -1.0, 3e9, -3e9])])
+    x = np.stack([v, v[::-1]], axis=1).astype(np.float32)
+    assert np.array_equal(encode(x, np.eye(2, dtype=np.float32), None, kout),
+                          oracle_lib.pca_encode(x, np.eye(2, dtype=np.float32), np.zeros(2, np.float32), kout))
