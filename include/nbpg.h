@@ -298,9 +298,10 @@ nbpg_status nbpg_gt(uint32_t dtype, uint32_t metric, uint32_t dims, const void *
                     const void *queries, uint32_t nq, uint32_t k, uint32_t mode, uint32_t *out_ids,
                     float *out_dists, int32_t device);
 
-/* Distance engine for nbpg_gt_with_engine: AUTO picks TENSOR where it applies (row length
- * up to 128 codes after 4-bit expansion, k <= 100) and DP4A otherwise; TENSOR on an
- * unsupported shape returns NBPG_ERR_UNSUPPORTED.  Results are identical across engines. */
+/* Distance engine for nbpg_gt_with_engine: AUTO picks the tensor engine where it applies (row
+ * length up to 640 codes after 4-bit expansion, k <= 128) and DP4A otherwise; TENSOR takes rows
+ * of up to 128 codes and k <= 100 and returns NBPG_ERR_UNSUPPORTED past that.  Results are
+ * identical across engines. */
 typedef enum nbpg_gt_engine { NBPG_GT_AUTO = 0, NBPG_GT_DP4A = 1, NBPG_GT_TENSOR = 2 } nbpg_gt_engine;
 
 nbpg_status nbpg_gt_with_engine(uint32_t dtype, uint32_t metric, uint32_t dims, const void *base, uint64_t n,
@@ -313,9 +314,10 @@ nbpg_status nbpg_gt_with_engine(uint32_t dtype, uint32_t metric, uint32_t dims, 
  * nbpg_gt_workspace_size() bytes of device workspace (0 for DP4A); d_workspace NULL
  * makes the call allocate it.  The size depends on the current device's SM count: the
  * tensor engine cuts the scans into one range per SM and keeps, per range and query, a list
- * of up to max(2048, 80 k rounded up to a power of two) candidates (1.5 GB on 152 SMs at
- * k = 100, besides the bf16 copies of base and queries).  Returns after the work has
- * finished on `stream`. */
+ * of up to 4,096 candidates (1.6 GB on 152 SMs for 10k queries at k = 100, besides the bf16
+ * copies of base and queries).  With AUTO, rows or k past the TENSOR limits also run where the
+ * workspace is smaller than that or cannot be allocated (the call allocates its own, or takes
+ * DP4A).  Returns after the work has finished on `stream`. */
 nbpg_status nbpg_gt_workspace_size(uint32_t dtype, uint32_t dims, uint64_t n, uint32_t nq, uint32_t k,
                                    uint32_t engine, size_t *bytes);
 nbpg_status nbpg_gt_device(uint32_t dtype, uint32_t metric, uint32_t dims, uint32_t row_stride, const void *d_base,

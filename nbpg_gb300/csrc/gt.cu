@@ -282,8 +282,13 @@ static cudaError_t launch_gt(const GtArgs &a, size_t smem, cudaStream_t st)
 bool gt_tc_supported(uint32_t dtype, uint32_t dims, uint32_t k, size_t smem_optin);
 nbpg_status gt_tc_device(uint32_t dtype, uint32_t metric, uint32_t dims, uint32_t stride, const uint8_t *d_base,
                          uint64_t n, const uint8_t *d_q, uint32_t nq, uint32_t k, uint32_t mode, uint32_t *d_ids,
-                         float *d_dists, void *ws, cudaStream_t st, bool withhold = false);
+                         float *d_dists, void *ws, cudaStream_t st);
 size_t gt_tc_workspace(uint32_t dtype, uint32_t dims, uint64_t n, uint32_t nq, uint32_t k);
+bool gt_scan_supported(uint32_t dtype, uint32_t dims, uint32_t k, size_t smem_optin);
+nbpg_status gt_scan_device(uint32_t dtype, uint32_t metric, uint32_t dims, uint32_t stride, const uint8_t *d_base,
+                           uint64_t n, const uint8_t *d_q, uint32_t nq, uint32_t k, uint32_t mode, uint32_t *d_ids,
+                           float *d_dists, void *ws, cudaStream_t st, bool *overflow, bool withhold = false);
+size_t gt_scan_workspace(uint32_t dtype, uint32_t dims, uint64_t n, uint32_t nq, uint32_t k);
 
 nbpg_status gt_device(uint32_t dtype, uint32_t metric, const GtArgs &a, cudaStream_t st, size_t smem_optin)
 {
@@ -314,6 +319,56 @@ nbpg_status gt_device(uint32_t dtype, uint32_t metric, const GtArgs &a, cudaStre
 
 using namespace nbpg;
 
+// What a call runs: the staged tensor scan (gt_scan.cu), with the replaying tensor engine (gt_tc.cu)
+// behind it for record lists that overflow, or DP4A.
+struct GtPlan {
+    bool scan;    // the staged scan
+    bool replay;  // the replaying tensor engine takes this shape (rows of up to 128 codes, k <= 100)
+    size_t smem_optin;
+};
+
+// TENSOR keeps the limits of the replaying engine; AUTO takes the staged scan wherever it applies.
+static nbpg_status resolve_engine(uint32_t dtype, uint32_t dims, uint32_t k, uint32_t engine, GtPlan *out)
+{
+    int dev = 0, optin = 0;
+    NBPG_CUDA_TRY(cudaGetDevice(&dev));
+    NBPG_CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    out->smem_optin = size_t(optin);
+    out->replay = gt_tc_supported(dtype, dims, k, size_t(optin));
+    out->scan = engine != NBPG_GT_DP4A && gt_scan_supported(dtype, dims, k, size_t(optin));
+    if (engine == NBPG_GT_TENSOR && !(out->replay && out->scan)) {
+        set_error("nbpg_gt: the tensor engine needs <= 128 codes per row and k <= 100");
+        return NBPG_ERR_UNSUPPORTED;
+    }
+    return NBPG_OK;
+}
+
+static size_t plan_workspace(const GtPlan &p, uint32_t dtype, uint32_t dims, uint64_t n, uint32_t nq, uint32_t k)
+{
+    if (!p.scan) return 0;
+    const size_t scan = gt_scan_workspace(dtype, dims, n, nq, k);
+    return p.replay ? std::max(scan, gt_tc_workspace(dtype, dims, n, nq, k)) : scan;
+}
+
+// Runs the plan; returns when the work is done or, for DP4A, enqueued.  ws holds plan_workspace()
+// bytes, or is NULL: the tensor engines then allocate theirs, and where DP4A alone used to run
+// (longer rows, larger k) it still does if that memory is not to be had.
+static nbpg_status run_plan(const GtPlan &p, uint32_t dtype, uint32_t metric, uint32_t dims, const GtArgs &a, uint32_t mode,
+                            void *ws, cudaStream_t st)
+{
+    if (p.scan) {
+        bool overflow = false;
+        const nbpg_status s = gt_scan_device(dtype, metric, dims, a.row_stride, a.base, a.n, a.queries, a.nq, a.k, mode,
+                                             a.out_ids, a.out_dists, ws, st, &overflow);
+        if (s == NBPG_OK && !overflow) return s;
+        if (s != NBPG_OK && !(s == NBPG_ERR_OOM && !p.replay)) return s;
+        if (p.replay)
+            return gt_tc_device(dtype, metric, dims, a.row_stride, a.base, a.n, a.queries, a.nq, a.k, mode, a.out_ids,
+                                a.out_dists, ws, st);
+    }
+    return gt_device(dtype, metric, a, st, p.smem_optin);
+}
+
 extern "C" nbpg_status nbpg_gt(uint32_t dtype, uint32_t metric, uint32_t dims, const void *base, uint64_t n,
                                const void *queries, uint32_t nq, uint32_t k, uint32_t mode, uint32_t *out_ids,
                                float *out_dists, int32_t device)
@@ -336,8 +391,6 @@ extern "C" nbpg_status nbpg_gt_with_engine(uint32_t dtype, uint32_t metric, uint
     NBPG_CUDA_TRY(cudaSetDevice(device));
     const uint32_t rb = dims;  // packed bytes per row (u8/i8/u4/i4)
     const uint32_t rs = round_up(rb, 16);
-    cudaDeviceProp prop{};
-    NBPG_CUDA_TRY(cudaGetDeviceProperties(&prop, device));
     cudaStream_t st;
     NBPG_CUDA_TRY(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
     uint8_t *db = nullptr, *dq = nullptr;
@@ -357,16 +410,11 @@ extern "C" nbpg_status nbpg_gt_with_engine(uint32_t dtype, uint32_t metric, uint
     if (e == cudaSuccess) e = cudaMemcpy2DAsync(db, rs, base, rb, rb, n, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpy2DAsync(dq, rs, queries, rb, rb, nq, cudaMemcpyHostToDevice, st);
     if (e != cudaSuccess) fail(e);
-    const bool tc_ok = gt_tc_supported(dtype, dims, k, prop.sharedMemPerBlockOptin);
-    if (s == NBPG_OK && engine == NBPG_GT_TENSOR && !tc_ok) {
-        set_error("nbpg_gt: the tensor engine needs <= 128 codes per row and k <= 100");
-        s = NBPG_ERR_UNSUPPORTED;
-    }
-    if (s == NBPG_OK && engine != NBPG_GT_DP4A && tc_ok) {
-        s = gt_tc_device(dtype, metric, dims, rs, db, n, dq, nq, k, mode, di, dd, nullptr, st);
-    } else if (s == NBPG_OK) {
-        GtArgs a{db, n, rs, dq, nq, k, mode == NBPG_GT_EXACT ? 1u : 0u, di, dd};
-        s = gt_device(dtype, metric, a, st, prop.sharedMemPerBlockOptin);
+    GtPlan plan{};
+    if (s == NBPG_OK) s = resolve_engine(dtype, dims, k, engine, &plan);
+    if (s == NBPG_OK) {
+        const GtArgs a{db, n, rs, dq, nq, k, mode == NBPG_GT_EXACT ? 1u : 0u, di, dd};
+        s = run_plan(plan, dtype, metric, dims, a, mode, nullptr, st);
     }
     if (s == NBPG_OK) {
         e = cudaMemcpyAsync(out_ids, di, size_t(nq) * k * 4, cudaMemcpyDeviceToHost, st);
@@ -383,31 +431,15 @@ extern "C" nbpg_status nbpg_gt_with_engine(uint32_t dtype, uint32_t metric, uint
     return s;
 }
 
-// Engine that a call with these arguments runs (AUTO resolved), or NBPG_ERR_UNSUPPORTED.
-static nbpg_status resolve_engine(uint32_t dtype, uint32_t dims, uint32_t k, uint32_t engine, uint32_t *out)
-{
-    int dev = 0;
-    NBPG_CUDA_TRY(cudaGetDevice(&dev));
-    int optin = 0;
-    NBPG_CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    const bool tc_ok = gt_tc_supported(dtype, dims, k, size_t(optin));
-    if (engine == NBPG_GT_TENSOR && !tc_ok) {
-        set_error("nbpg_gt: the tensor engine needs <= 128 codes per row and k <= 100");
-        return NBPG_ERR_UNSUPPORTED;
-    }
-    *out = (engine != NBPG_GT_DP4A && tc_ok) ? uint32_t(NBPG_GT_TENSOR) : uint32_t(NBPG_GT_DP4A);
-    return NBPG_OK;
-}
-
 extern "C" nbpg_status nbpg_gt_workspace_size(uint32_t dtype, uint32_t dims, uint64_t n, uint32_t nq, uint32_t k,
                                               uint32_t engine, size_t *bytes)
 {
     NBPG_CHECK_ARG(bytes, "null argument");
     NBPG_CHECK_ARG(dtype <= NBPG_I4 && dims >= 1 && engine <= NBPG_GT_TENSOR, "bad dtype/dims/engine");
-    uint32_t eng = 0;
-    const nbpg_status s = resolve_engine(dtype, dims, k, engine, &eng);
+    GtPlan plan{};
+    const nbpg_status s = resolve_engine(dtype, dims, k, engine, &plan);
     if (s != NBPG_OK) return s;
-    *bytes = eng == NBPG_GT_TENSOR ? gt_tc_workspace(dtype, dims, n, nq, k) : 0;
+    *bytes = plan_workspace(plan, dtype, dims, n, nq, k);
     return NBPG_OK;
 }
 
@@ -425,22 +457,16 @@ extern "C" nbpg_status nbpg_gt_device(uint32_t dtype, uint32_t metric, uint32_t 
     NBPG_CHECK_ARG((reinterpret_cast<uintptr_t>(d_base) | reinterpret_cast<uintptr_t>(d_queries)) % 16 == 0,
                    "base and queries must be 16-byte aligned");
     if (nq == 0) return NBPG_OK;
-    uint32_t eng = 0;
-    nbpg_status s = resolve_engine(dtype, dims, k, engine, &eng);
+    GtPlan plan{};
+    nbpg_status s = resolve_engine(dtype, dims, k, engine, &plan);
     if (s != NBPG_OK) return s;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (eng == NBPG_GT_TENSOR) {
-        const size_t need = gt_tc_workspace(dtype, dims, n, nq, k);
-        NBPG_CHECK_ARG(!d_workspace || workspace_bytes >= need, "workspace smaller than nbpg_gt_workspace_size");
-        return gt_tc_device(dtype, metric, dims, row_stride, static_cast<const uint8_t *>(d_base), n,
-                            static_cast<const uint8_t *>(d_queries), nq, k, mode, d_ids, d_dists, d_workspace, st);
-    }
-    int dev = 0, optin = 0;
-    NBPG_CUDA_TRY(cudaGetDevice(&dev));
-    NBPG_CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    GtArgs a{static_cast<const uint8_t *>(d_base), n, row_stride, static_cast<const uint8_t *>(d_queries), nq, k,
-             mode == NBPG_GT_EXACT ? 1u : 0u, d_ids, d_dists};
-    s = gt_device(dtype, metric, a, st, size_t(optin));
+    const size_t need = plan_workspace(plan, dtype, dims, n, nq, k);
+    NBPG_CHECK_ARG(!plan.replay || !plan.scan || !d_workspace || workspace_bytes >= need,
+                   "workspace smaller than nbpg_gt_workspace_size");
+    const GtArgs a{static_cast<const uint8_t *>(d_base), n, row_stride, static_cast<const uint8_t *>(d_queries), nq, k,
+                   mode == NBPG_GT_EXACT ? 1u : 0u, d_ids, d_dists};
+    s = run_plan(plan, dtype, metric, dims, a, mode, workspace_bytes >= need ? d_workspace : nullptr, st);
     if (s == NBPG_OK) NBPG_CUDA_TRY(cudaStreamSynchronize(st));
     return s;
 }

@@ -1,5 +1,10 @@
-// Brute-force kNN with tcgen05 tensor cores: compute_groundtruth
+// Brute-force kNN with tcgen05 tensor cores, replaying as it scans: compute_groundtruth
 // (data_tools/ANNs/data_proc/CompGT.cpp:29-134), same outputs as gt.cu.
+//
+// Runs when a record list of the staged scan (gt_scan.cu) overflows: rows ordered so that thousands
+// in one range come closer and closer to a query.  Here most of those are admitted where they are
+// met, without a list.  On rows in random order the staged scan is the faster one (10k x 1M x 128,
+// k = 100: 4.2 ms against 9.6).
 //
 // Exactness: u8 (0..255), i8 (-128..127) and 4-bit codes are exact in bf16, their
 // products are exact in fp32, and every partial sum of a row's dot product stays an
@@ -21,7 +26,6 @@
 // that bound, and gt_tc_merge_kernel replays the records in id order after the first
 // segment's list.  All waits on mbarriers are bounded; on a timeout the kernel records an
 // error and tears down.
-#include <cuda.h>
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -30,17 +34,15 @@
 
 #include "common.cuh"
 #include "internal.h"
+#include "tc_util.cuh"
 
 namespace nbpg {
 
 constexpr int TC_M = 128;        // queries per CTA
 constexpr int TC_N = 128;        // base rows per tile
-constexpr int TC_KATOM = 64;     // bf16 elements per 128-byte swizzled row
 constexpr uint32_t TC_MAX_STAGES = 4;  // shared-memory ring of base tiles: 2..4 deep as memory allows
 constexpr uint32_t TC_ACC = 4;         // TMEM accumulators of 128 columns: all 512 columns of the SM
 constexpr int TC_THREADS = 192;  // warps 0-3 epilogue, 4 TMA, 5 MMA
-constexpr uint64_t TC_WAIT_NS = 2000000000ull;  // 2 s: far above any wait of a working pipeline
-constexpr uint32_t TC_WAIT_POLLS = 1u << 30;
 constexpr uint32_t TC_QUEUE = 8;  // flagged candidates queued per query before a drain
 
 struct TcArgs {
@@ -51,7 +53,6 @@ struct TcArgs {
     uint32_t katoms;               // K / 64
     uint32_t T;                    // base tiles of one full scan
     uint32_t stages;               // depth of the base-tile ring
-    uint32_t withhold;             // test hook: the producer issues no base tiles
     uint32_t *out_ids;             // slot-order lists after the scan, (dist, id)-sorted after the merge
     float *out_dists;
     uint32_t *err;
@@ -111,118 +112,6 @@ __host__ __device__ __forceinline__ TcSeg tc_seg_at(const TcRange &r, uint32_t i
 
 __device__ __forceinline__ float ld_volatile(const float *p) { return *reinterpret_cast<const volatile float *>(p); }
 __device__ __forceinline__ void st_volatile(float *p, float v) { *reinterpret_cast<volatile float *>(p) = v; }
-
-__device__ __forceinline__ uint32_t smem_u32(const void *p)
-{
-    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count)
-{
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
-}
-
-__device__ __forceinline__ void mbar_arrive(uint32_t bar)
-{
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes)
-{
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-
-__device__ __forceinline__ uint64_t global_ns()
-{
-    uint64_t t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
-// Bounded wait for the phase of the given parity; false (and *err set) when it has not
-// completed within TC_WAIT_NS of wall time (try_wait may itself suspend the thread for a
-// while, so the bound is on the clock, with a poll count as the last resort).
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_t *err)
-{
-    uint64_t t0 = 0;
-    for (uint32_t it = 0; it < TC_WAIT_POLLS; ++it) {
-        uint32_t done;
-        asm volatile(
-            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-            : "=r"(done)
-            : "r"(bar), "r"(parity)
-            : "memory");
-        if (done) return true;
-        if (it == 64) t0 = global_ns();
-        if (it > 64) {
-            __nanosleep(64);
-            if ((it & 255) == 0 && global_ns() - t0 > TC_WAIT_NS) break;
-        }
-    }
-    atomicExch(err, 1u);
-    return false;
-}
-
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, int32_t x, int32_t y, uint32_t bar)
-{
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::
-            "r"(dst),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar)
-        : "memory");
-}
-
-// plain bulk copy global -> shared (16-byte aligned, size a multiple of 16), completing on bar
-__device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar)
-{
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-                 "l"(src), "r"(bytes), "r"(bar)
-                 : "memory");
-}
-
-// K-major operand, 128-byte swizzle: rows of 128 B, 8-row groups 1024 B apart
-__device__ __forceinline__ uint64_t sw128_desc(uint32_t addr)
-{
-    uint64_t d = 0;
-    d |= uint64_t((addr & 0x3FFFFu) >> 4);
-    d |= uint64_t(1) << 16;             // leading byte offset (unused with 128-byte swizzle)
-    d |= uint64_t(1024 >> 4) << 32;     // stride byte offset: 8 rows x 128 B
-    d |= uint64_t(1) << 46;             // descriptor version
-    d |= uint64_t(2) << 61;             // 128-byte swizzle
-    return d;
-}
-
-// kind::f16 instruction descriptor: fp32 accumulator, bf16 A and B, both K-major
-__host__ __device__ constexpr uint32_t tc_idesc(uint32_t M, uint32_t N)
-{
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((N >> 3) << 17) | ((M >> 4) << 24);
-}
-
-__device__ __forceinline__ void tc_mma(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc)
-{
-    asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem_d),
-        "l"(a), "l"(b), "r"(idesc), "r"(acc));
-}
-
-__device__ __forceinline__ void tc_commit(uint32_t bar)
-{
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-
-__device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t (&v)[32])
-{
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,"
-        "%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-          "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]),
-          "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
-          "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-        : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
 
 // Per-query top-k list in shared memory, [k][128] so that thread t's entries stride 128,
 // with a tournament tree over list slots [lo, k) whose internal nodes (1 .. P-1, P the
@@ -506,7 +395,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                 for (uint32_t c = 0; c < a.katoms; ++c)
                     tma_load_2d(smem_u32(sA + c * atom_bytes), &tmA, int32_t(c * TC_KATOM), int32_t(qt * TC_M), bar_a);
                 ++aloads;
-                for (uint32_t b = g.b0; b < (a.withhold ? g.b0 : g.b1); ++b) {
+                for (uint32_t b = g.b0; b < g.b1; ++b) {
                     if (!mbar_wait(bar_empty + 8 * s, ph ^ 1, a.err)) {
                         ok = false;
                         break;
@@ -861,37 +750,6 @@ __global__ void __launch_bounds__(256) to_bf16_kernel(const uint8_t *src, uint32
     if (r < rows_pad && g == 0) norm[r] = float(acc);  // at most 128 * 255^2 < 2^24: exact
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
-                                  const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-static EncodeTiledFn encode_fn()
-{
-    static EncodeTiledFn fn = nullptr;
-    if (!fn) {
-        void *p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) ==
-                cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<EncodeTiledFn>(p);
-    }
-    return fn;
-}
-
-static bool make_map(CUtensorMap *m, void *base, uint64_t rows, uint32_t K)
-{
-    EncodeTiledFn enc = encode_fn();
-    if (!enc) return false;
-    const cuuint64_t dims[2] = {K, rows};
-    const cuuint64_t strides[1] = {uint64_t(K) * 2};
-    const cuuint32_t box[2] = {TC_KATOM, 128};
-    const cuuint32_t estr[2] = {1, 1};
-    return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 // Dynamic shared memory of one CTA with a ring of `stages` base tiles.  At least 120 KB,
 // so that one CTA holds an SM and its TMEM allocation (all 512 columns) never waits
 // for another's.
@@ -1030,7 +888,7 @@ size_t gt_tc_workspace(uint32_t dtype, uint32_t dims, uint64_t n, uint32_t nq, u
 // kernel has finished (the error flag of the bounded waits is read back).
 nbpg_status gt_tc_device(uint32_t dtype, uint32_t metric, uint32_t dims, uint32_t stride, const uint8_t *d_base,
                          uint64_t n, const uint8_t *d_q, uint32_t nq, uint32_t k, uint32_t mode, uint32_t *d_ids,
-                         float *d_dists, void *ws, cudaStream_t st, bool withhold = false)
+                         float *d_dists, void *ws, cudaStream_t st)
 {
     const bool nib = dtype == NBPG_U4 || dtype == NBPG_I4;
     const TcLayout l = tc_layout(dtype, dims, n, nq, k, device_sms());
@@ -1108,7 +966,6 @@ nbpg_status gt_tc_device(uint32_t dtype, uint32_t metric, uint32_t dims, uint32_
     a.katoms = l.katoms;
     a.T = uint32_t(n_pad / TC_N);
     a.stages = stages;
-    a.withhold = withhold ? 1u : 0u;
     a.out_ids = d_ids;
     a.out_dists = d_dists;
     a.err = err;
@@ -1204,36 +1061,4 @@ extern "C" nbpg_status nbpg_test_gt_split(uint32_t qtiles, uint32_t T, uint32_t 
         conts[2 * i + 1] = ct[i].y;
     }
     return NBPG_OK;
-}
-
-// Test hook for the failure path: the tensor kNN on a small problem with its base tiles
-// withheld, so the MMA and epilogue waits run out (nothing ever arrives on those barriers);
-// the kernel must record the timeout, tear down (final commit, TMEM freed) and return, and
-// the context must stay usable.  Returns NBPG_ERR_TIMEOUT on that path.
-extern "C" nbpg_status nbpg_test_gt_timeout(int32_t device)
-{
-    using namespace nbpg;
-    NBPG_CUDA_TRY(cudaSetDevice(device));
-    const uint32_t n = 512, nq = 128, dims = 64, k = 10;
-    uint8_t *db = nullptr, *dq = nullptr;
-    uint32_t *di = nullptr;
-    float *dd = nullptr;
-    cudaError_t e = cudaMalloc(&db, n * dims);
-    if (e == cudaSuccess) e = cudaMalloc(&dq, nq * dims);
-    if (e == cudaSuccess) e = cudaMalloc(&di, nq * k * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&dd, nq * k * 4);
-    if (e == cudaSuccess) e = cudaMemset(db, 7, n * dims);
-    if (e == cudaSuccess) e = cudaMemset(dq, 3, nq * dims);
-    nbpg_status s = NBPG_ERR_CUDA;
-    if (e == cudaSuccess) s = gt_tc_device(NBPG_U8, NBPG_L2, dims, dims, db, n, dq, nq, k, NBPG_GT_COMPGT, di, dd,
-                                           nullptr, nullptr, true);
-    cudaFree(db);
-    cudaFree(dq);
-    cudaFree(di);
-    cudaFree(dd);
-    if (e != cudaSuccess) {
-        set_error(std::string("nbpg_test_gt_timeout: ") + cudaGetErrorString(e));
-        return NBPG_ERR_CUDA;
-    }
-    return s;
 }

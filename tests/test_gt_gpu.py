@@ -166,3 +166,61 @@ def test_tensor_engine_timeout_path(gpu_lib, oracle_lib):
     ids, ds = ground_truth(b, q, "u8", "l2", k=10, engine="tensor")
     oi, od = oracle_lib.gt("u8", "l2", b, q, k=10)
     assert np.array_equal(ids, oi) and np.array_equal(ds, od)
+
+
+@pytest.mark.parametrize("dtype,dims,n,nq,k", [
+    ("u8", 129, 3000, 5, 10), ("u8", 192, 5000, 257, 100), ("u8", 193, 2500, 40, 128), ("i8", 256, 4000, 129, 17),
+    ("u8", 257, 1500, 128, 101), ("i8", 320, 1100, 130, 1), ("u8", 511, 2000, 33, 49), ("u8", 640, 6000, 300, 100),
+    ("u8", 641, 1300, 7, 10), ("u4", 65, 4000, 100, 50), ("i4", 129, 2000, 20, 10), ("u4", 320, 3000, 64, 100),
+    ("u8", 64, 1024, 256, 128), ("i8", 65, 1025, 1, 128), ("u8", 16, 128, 3, 128), ("u8", 8, 4097, 300, 16)])
+@pytest.mark.parametrize("metric", ["l2", "ip"])
+def test_gt_auto_long_rows(gpu_lib, oracle_lib, dtype, dims, n, nq, k, metric):
+    """AUTO past the 128 codes / 100 neighbours of the explicit tensor engine: one and two query
+    tiles per CTA, every number of 64-code columns up to 640 codes and the first row past it, k up
+    to 128, sums that pass 2^24 (extreme codes), stage and tile edges, ties."""
+    from nbpg_gb300.index import ground_truth
+    r = np.random.default_rng(dims * 7 + n)
+    if dtype == "u8":  # half of the codes at the ends of the range: the largest distances there are
+        x = np.where(r.random((n + nq, dims)) < 0.5, r.choice([0, 255], (n + nq, dims)), r.integers(0, 256, (n + nq, dims)))
+        x = x.astype(np.uint8)
+    elif dtype == "i8":
+        x = r.integers(-128, 128, (n + nq, dims)).astype(np.int8)
+    else:
+        x = r.integers(0, 256, (n + nq, dims)).astype(np.uint8)
+    base, q = np.ascontiguousarray(x[:n]), np.ascontiguousarray(x[n:])
+    base[n // 2:n // 2 + 20] = base[:20]  # repeated rows: equal distances, order by id
+    for exact in (False, True):
+        ids, ds = ground_truth(base, q, dtype, metric, k=k, exact=exact)
+        oi, od = oracle_lib.gt(dtype, metric, base, q, k=k, exact=exact)
+        assert np.array_equal(ids, oi), exact
+        assert np.array_equal(ds.view(np.uint32), od.view(np.uint32)), exact
+
+
+@pytest.mark.parametrize("exact", [False, True])
+def test_gt_stages_against_dp4a(gpu_lib, exact):
+    """Several query batches (more than 64 tiles of 256), many stages, one query over many ranges:
+    the staged scan equals the DP4A engine."""
+    from nbpg_gb300 import synth
+    from nbpg_gb300.index import ground_truth
+    b, q = synth.u8_mixture(70001, 16700, dim=24, n_centres=64)
+    for n, nq, k in [(9000, 16700, 10), (70001, 1, 100), (70001, 700, 33)]:
+        a = ground_truth(b[:n], q[:nq], "u8", "l2", k=k, exact=exact)
+        d = ground_truth(b[:n], q[:nq], "u8", "l2", k=k, exact=exact, engine="dp4a")
+        assert np.array_equal(a[0], d[0]) and np.array_equal(a[1], d[1]), (n, nq, k)
+
+
+@pytest.mark.parametrize("dims", [16, 136])
+def test_gt_record_overflow(gpu_lib, dims):
+    """Rows that come closer and closer, more of them per range than a record list holds (12 query
+    tiles x 3,000 base tiles on about 152 ranges): the call goes on to an engine without lists (the
+    replaying tensor engine for short rows, DP4A for long ones) and stays exact."""
+    from nbpg_gb300.index import ground_truth
+    r = np.random.default_rng(9)
+    b = r.integers(0, 256, (384000, dims)).astype(np.uint8)
+    b = np.ascontiguousarray(b[np.argsort(-(b.astype(np.int32) ** 2).sum(1), kind="stable")])
+    q = np.zeros((3000, dims), np.uint8)
+    q[::2, 0] = 1
+    for exact in (False, True):
+        a = ground_truth(b, q, "u8", "l2", k=10, exact=exact)
+        d = ground_truth(b, q, "u8", "l2", k=10, exact=exact, engine="dp4a")
+        assert np.array_equal(a[0], d[0]) and np.array_equal(a[1], d[1]), exact
