@@ -64,6 +64,24 @@ SlotLayout make_slot_layout(uint32_t Lmax, uint32_t R, bool vis_smem, uint32_t V
     return l;
 }
 
+// Per-warp slot of search_flag: the query row, one frontier, candidates, the filter, filtered ids.
+SlotLayout make_flag_layout(uint32_t Lmax, uint32_t R, uint32_t row_stride, bool hash_smem, uint32_t Scap)
+{
+    SlotLayout l{};
+    l.Lcap = round_up(std::max<uint32_t>(Lmax, 1), 32);
+    l.Ccap = round_up(l.Lcap / 8 + R + 1, 32);
+    l.Rcap = round_up(std::max<uint32_t>(R, 1), 32);
+    l.Scap = hash_smem ? Scap : 0;
+    uint32_t off = 0;
+    l.off_q = off; off += row_stride;
+    l.off_fr0 = off; off += l.Lcap * 8;
+    l.off_cand = off; off += l.Ccap * 8;
+    l.off_hash = off; off += l.Scap * 4;
+    l.off_filt = off; off += l.Rcap * 4;
+    l.bytes = round_up(off, 16);
+    return l;
+}
+
 // Thresholds for keeping per-query tables in shared memory.
 static constexpr uint32_t kHashSmemMax = 32768;  // bytes of visited filter per warp slot
 static constexpr uint32_t kVisSmemMax = 16384;   // bytes of visited list per warp slot
@@ -81,54 +99,56 @@ struct PassCfg {
 // time than a 10k-query search spends on the device).  The dynamic shared-memory attribute of a
 // kernel is only ever raised, so every cached plan stays launchable.
 static std::mutex g_plan_mu;
-using PlanKey = std::tuple<int, const SearchOps *, int, bool, bool, uint32_t, uint32_t, uint32_t, uint32_t, size_t, int>;
+using PlanKey = std::tuple<int, const SearchOps *, int, int, bool, uint32_t, uint32_t, uint32_t, uint32_t, size_t, int, uint32_t>;
 static std::map<PlanKey, PassCfg> g_plans;
-static std::map<std::tuple<int, const SearchOps *, int, bool, bool>, size_t> g_attr;
+static std::map<std::tuple<int, const SearchOps *, int, int, bool>, size_t> g_attr;
 
-static cudaError_t raise_attr(int device, const SearchOps *ops, int metric, bool list, bool plain, size_t smem)
+static cudaError_t raise_attr(int device, const SearchOps *ops, int metric, int pass, bool plain, size_t smem)
 {
-    size_t &cur = g_attr[std::make_tuple(device, ops, metric, list, plain)];
+    size_t &cur = g_attr[std::make_tuple(device, ops, metric, pass, plain)];
     if (smem <= cur) return cudaSuccess;
-    const cudaError_t e = ops->set_attr(metric, list, plain, smem);
+    const cudaError_t e = ops->set_attr(metric, pass, plain, smem);
     if (e == cudaSuccess) cur = smem;
     return e;
 }
 
-cudaError_t raise_search_attr(int device, const SearchOps *ops, int metric, bool list, bool plain, size_t smem)
+cudaError_t raise_search_attr(int device, const SearchOps *ops, int metric, int pass, bool plain, size_t smem)
 {
     std::lock_guard<std::mutex> g(g_plan_mu);
-    return raise_attr(device, ops, metric, list, plain, smem);
+    return raise_attr(device, ops, metric, pass, plain, smem);
 }
 
-static nbpg_status plan_pass_uncached(nbpg_index *idx, const SearchOps *ops, int metric, bool list, bool plain,
+static nbpg_status plan_pass_uncached(nbpg_index *idx, const SearchOps *ops, int metric, int pass, bool plain,
                                       uint32_t Lmax, uint32_t vf, uint32_t want_warps, PassCfg &pc);
 
-static nbpg_status plan_pass(nbpg_index *idx, const SearchOps *ops, int metric, bool list, bool plain, uint32_t Lmax,
+static nbpg_status plan_pass(nbpg_index *idx, const SearchOps *ops, int metric, int pass, bool plain, uint32_t Lmax,
                              uint32_t vf, uint32_t want_warps, PassCfg &pc)
 {
-    const PlanKey key{idx->desc.device, ops, metric, list, plain, Lmax, vf, want_warps, idx->desc.max_degree,
-                      idx->smem_optin, idx->sm_count};
+    const PlanKey key{idx->desc.device, ops, metric, pass, plain, Lmax, vf, want_warps, idx->desc.max_degree,
+                      idx->smem_optin, idx->sm_count, idx->row_stride};
     std::lock_guard<std::mutex> g(g_plan_mu);
     auto it = g_plans.find(key);
     if (it != g_plans.end()) {
         pc = it->second;
         return NBPG_OK;
     }
-    const nbpg_status s = plan_pass_uncached(idx, ops, metric, list, plain, Lmax, vf, want_warps, pc);
+    const nbpg_status s = plan_pass_uncached(idx, ops, metric, pass, plain, Lmax, vf, want_warps, pc);
     if (s == NBPG_OK) g_plans.emplace(key, pc);
     return s;
 }
 
-static nbpg_status plan_pass_uncached(nbpg_index *idx, const SearchOps *ops, int metric, bool list, bool plain,
+static nbpg_status plan_pass_uncached(nbpg_index *idx, const SearchOps *ops, int metric, int pass, bool plain,
                                       uint32_t Lmax, uint32_t vf, uint32_t want_warps, PassCfg &pc)
 {
     const int dev = idx->desc.device;
     const uint32_t R = idx->desc.max_degree;
+    const bool list = pass == PASS_LIST;
     pc.S = filter_slots_for(Lmax);
     pc.Vcap = round_up(vf * Lmax, 32);
     pc.ghash = !plain && pc.S * 4 > kHashSmemMax;
     pc.gvis = list && !plain && pc.Vcap * 8 > kVisSmemMax;
-    pc.lay = make_slot_layout(Lmax, R, list && !pc.gvis, pc.Vcap, !pc.ghash, pc.S);
+    pc.lay = pass == PASS_WIDE ? make_flag_layout(Lmax, R, idx->row_stride, !pc.ghash, pc.S)
+                               : make_slot_layout(Lmax, R, list && !pc.gvis, pc.Vcap, !pc.ghash, pc.S);
     if (pc.lay.bytes > idx->smem_optin) {
         set_error("per-query working set exceeds shared memory for this L");
         return NBPG_ERR_UNSUPPORTED;
@@ -136,7 +156,7 @@ static nbpg_status plan_pass_uncached(nbpg_index *idx, const SearchOps *ops, int
     if (plain) {
         pc.warps = 1;
         pc.smem = pc.lay.bytes;
-        NBPG_CUDA_TRY(raise_attr(dev, ops, metric, list, true, pc.smem));
+        NBPG_CUDA_TRY(raise_attr(dev, ops, metric, pass, true, pc.smem));
         return NBPG_OK;
     }
     uint32_t fit = uint32_t(idx->smem_optin / pc.lay.bytes);
@@ -149,8 +169,8 @@ static nbpg_status plan_pass_uncached(nbpg_index *idx, const SearchOps *ops, int
             if (c > fit) continue;
             const size_t sm = size_t(c) * pc.lay.bytes;
             int b = 0;
-            NBPG_CUDA_TRY(raise_attr(dev, ops, metric, list, false, sm));
-            NBPG_CUDA_TRY(ops->occ(metric, list, false, int(c) * 32, sm, &b));
+            NBPG_CUDA_TRY(raise_attr(dev, ops, metric, pass, false, sm));
+            NBPG_CUDA_TRY(ops->occ(metric, pass, false, int(c) * 32, sm, &b));
             if (int(c) * b > best) { best = int(c) * b; w = c; }
         }
         if (!w) w = 1;
@@ -158,9 +178,9 @@ static nbpg_status plan_pass_uncached(nbpg_index *idx, const SearchOps *ops, int
     w = std::max<uint32_t>(1, std::min<uint32_t>(w, std::min<uint32_t>(16, fit)));
     pc.warps = w;
     pc.smem = size_t(w) * pc.lay.bytes;
-    NBPG_CUDA_TRY(raise_attr(dev, ops, metric, list, false, pc.smem));
+    NBPG_CUDA_TRY(raise_attr(dev, ops, metric, pass, false, pc.smem));
     int blocks = 0;
-    NBPG_CUDA_TRY(ops->occ(metric, list, false, w * 32, pc.smem, &blocks));
+    NBPG_CUDA_TRY(ops->occ(metric, pass, false, w * 32, pc.smem, &blocks));
     if (blocks < 1) {
         set_error("search kernel does not fit on an SM");
         return NBPG_ERR_UNSUPPORTED;
@@ -377,10 +397,12 @@ nbpg_status search_device_impl(nbpg_index *idx, SearchScratch &sc, const void *d
                        "k_stride must hold the visited list (visited_factor * L)");
 
     PassCfg main{}, rerun{};
-    nbpg_status s = plan_pass(idx, ops, metric, !flag_first, plain, P->L, vf, P->warps_per_cta, main);
+    // beams above 32 (the largest of the call): search_flag's merge, several frontier words
+    const int pass = !flag_first ? PASS_LIST : P->L > 32 ? PASS_WIDE : PASS_FLAG;
+    nbpg_status s = plan_pass(idx, ops, metric, pass, plain, P->L, vf, P->warps_per_cta, main);
     if (s != NBPG_OK) return s;
     if (flag_first) {
-        s = plan_pass(idx, ops, metric, true, false, P->L, vf, 0, rerun);
+        s = plan_pass(idx, ops, metric, PASS_LIST, false, P->L, vf, 0, rerun);
         if (s != NBPG_OK) return s;
     }
 
@@ -452,7 +474,7 @@ nbpg_status search_device_impl(nbpg_index *idx, SearchScratch &sc, const void *d
     m.g_hash_slots = main.ghash ? hslots : 0;
     m.g_vis = main.gvis ? sc.gvis.as<uint64_t>() : nullptr;
     m.g_vis_cap = main.gvis ? vcap : 0;
-    ops->launch(metric, !flag_first, plain, plain ? nq : main.grid, main.warps, main.smem, m, st);
+    ops->launch(metric, pass, plain, plain ? nq : main.grid, main.warps, main.smem, m, st);
     NBPG_CUDA_TRY(cudaGetLastError());
 
     if (flag_first) {
@@ -465,7 +487,7 @@ nbpg_status search_device_impl(nbpg_index *idx, SearchScratch &sc, const void *d
         r.g_vis = rerun.gvis ? sc.gvis.as<uint64_t>() : nullptr;
         r.g_vis_cap = rerun.gvis ? vcap : 0;
         r.prefetch = 0;
-        ops->launch(metric, true, false, rerun.grid, rerun.warps, rerun.smem, r, st);
+        ops->launch(metric, PASS_LIST, false, rerun.grid, rerun.warps, rerun.smem, r, st);
         NBPG_CUDA_TRY(cudaGetLastError());
     }
     return NBPG_OK;

@@ -2,6 +2,7 @@
 #pragma once
 #include "internal.h"
 #include "search_fast.cuh"
+#include "search_kernels.cuh"
 
 namespace nbpg {
 
@@ -18,28 +19,28 @@ struct LaunchPlan {
     bool ghash_main, ghash_list, gvis_list;
 };
 
-template <int DT, int MET, bool LIST, int VPL>
+template <int DT, int MET, int PASS, int VPL>
 inline cudaError_t set_smem_attr(bool plain, size_t smem)
 {
     if (plain)
-        return cudaFuncSetAttribute(search_plain_kernel<DT, MET, LIST, VPL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        return cudaFuncSetAttribute(search_plain_kernel<DT, MET, PASS, VPL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     int(smem));
-    return cudaFuncSetAttribute(search_batched_kernel<DT, MET, LIST, VPL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    return cudaFuncSetAttribute(search_batched_kernel<DT, MET, PASS, VPL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 int(smem));
 }
 
-template <int DT, int MET, bool LIST, int VPL>
+template <int DT, int MET, int PASS, int VPL>
 inline cudaError_t occupancy(bool plain, uint32_t threads, size_t smem, int *blocks)
 {
-    if (plain) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, search_plain_kernel<DT, MET, LIST, VPL>, int(threads), smem);
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, search_batched_kernel<DT, MET, LIST, VPL>, int(threads), smem);
+    if (plain) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, search_plain_kernel<DT, MET, PASS, VPL>, int(threads), smem);
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, search_batched_kernel<DT, MET, PASS, VPL>, int(threads), smem);
 }
 
-template <int DT, int MET, bool LIST, int VPL>
+template <int DT, int MET, int PASS, int VPL>
 inline void launch_one(bool plain, uint32_t grid, uint32_t warps, size_t smem, const SearchArgs &a, cudaStream_t st)
 {
-    if (plain) search_plain_kernel<DT, MET, LIST, VPL><<<grid, 32, smem, st>>>(a);
-    else search_batched_kernel<DT, MET, LIST, VPL><<<grid, warps * 32, smem, st>>>(a);
+    if (plain) search_plain_kernel<DT, MET, PASS, VPL><<<grid, 32, smem, st>>>(a);
+    else search_batched_kernel<DT, MET, PASS, VPL><<<grid, warps * 32, smem, st>>>(a);
 }
 
 template <int DT, int MET, int VPL>
@@ -73,30 +74,27 @@ inline void launch_fast_one(bool plain, uint32_t grid, uint32_t warps, size_t sm
 // Dispatch on (metric, mode) for one element type and lane width.
 template <int DT, int VPL>
 struct SearchDispatch {
-    static cudaError_t set_attr(int metric, bool list, bool plain, size_t smem)
+    static cudaError_t set_attr(int metric, int pass, bool plain, size_t smem)
     {
-        if (metric == M_L2)
-            return list ? set_smem_attr<DT, M_L2, true, VPL>(plain, smem) : set_smem_attr<DT, M_L2, false, VPL>(plain, smem);
-        return list ? set_smem_attr<DT, M_IP, true, VPL>(plain, smem) : set_smem_attr<DT, M_IP, false, VPL>(plain, smem);
+        if (metric == M_IP) return set_smem_attr<DT, M_IP, PASS_LIST, VPL>(plain, smem);
+        if (pass == PASS_LIST) return set_smem_attr<DT, M_L2, PASS_LIST, VPL>(plain, smem);
+        return pass == PASS_WIDE ? set_smem_attr<DT, M_L2, PASS_WIDE, VPL>(plain, smem)
+                                 : set_smem_attr<DT, M_L2, PASS_FLAG, VPL>(plain, smem);
     }
-    static cudaError_t occ(int metric, bool list, bool plain, uint32_t threads, size_t smem, int *blocks)
+    static cudaError_t occ(int metric, int pass, bool plain, uint32_t threads, size_t smem, int *blocks)
     {
-        if (metric == M_L2)
-            return list ? occupancy<DT, M_L2, true, VPL>(plain, threads, smem, blocks)
-                        : occupancy<DT, M_L2, false, VPL>(plain, threads, smem, blocks);
-        return list ? occupancy<DT, M_IP, true, VPL>(plain, threads, smem, blocks)
-                    : occupancy<DT, M_IP, false, VPL>(plain, threads, smem, blocks);
+        if (metric == M_IP) return occupancy<DT, M_IP, PASS_LIST, VPL>(plain, threads, smem, blocks);
+        if (pass == PASS_LIST) return occupancy<DT, M_L2, PASS_LIST, VPL>(plain, threads, smem, blocks);
+        return pass == PASS_WIDE ? occupancy<DT, M_L2, PASS_WIDE, VPL>(plain, threads, smem, blocks)
+                                 : occupancy<DT, M_L2, PASS_FLAG, VPL>(plain, threads, smem, blocks);
     }
-    static void launch(int metric, bool list, bool plain, uint32_t grid, uint32_t warps, size_t smem,
-                       const SearchArgs &a, cudaStream_t st)
+    static void launch(int metric, int pass, bool plain, uint32_t grid, uint32_t warps, size_t smem, const SearchArgs &a,
+                       cudaStream_t st)
     {
-        if (metric == M_L2) {
-            if (list) launch_one<DT, M_L2, true, VPL>(plain, grid, warps, smem, a, st);
-            else launch_one<DT, M_L2, false, VPL>(plain, grid, warps, smem, a, st);
-        } else {
-            if (list) launch_one<DT, M_IP, true, VPL>(plain, grid, warps, smem, a, st);
-            else launch_one<DT, M_IP, false, VPL>(plain, grid, warps, smem, a, st);
-        }
+        if (metric == M_IP) launch_one<DT, M_IP, PASS_LIST, VPL>(plain, grid, warps, smem, a, st);
+        else if (pass == PASS_LIST) launch_one<DT, M_L2, PASS_LIST, VPL>(plain, grid, warps, smem, a, st);
+        else if (pass == PASS_WIDE) launch_one<DT, M_L2, PASS_WIDE, VPL>(plain, grid, warps, smem, a, st);
+        else launch_one<DT, M_L2, PASS_FLAG, VPL>(plain, grid, warps, smem, a, st);
     }
     static cudaError_t set_attr_fast(int metric, bool plain, size_t smem)
     {

@@ -210,17 +210,17 @@ extern "C" nbpg_status nbpg_search_noalloc(uint32_t dtype, uint32_t metric, uint
                 if (c > fit) continue;
                 const size_t sm = size_t(c) * lay.bytes;
                 int b = 0;
-                NBPG_CUDA_TRY(raise_search_attr(device, ops, met, list, false, sm));
-                NBPG_CUDA_TRY(ops->occ(met, list, false, int(c) * 32, sm, &b));
+                NBPG_CUDA_TRY(raise_search_attr(device, ops, met, list ? PASS_LIST : PASS_FLAG, false, sm));
+                NBPG_CUDA_TRY(ops->occ(met, list ? PASS_LIST : PASS_FLAG, false, int(c) * 32, sm, &b));
                 if (int(c) * b > best) { best = int(c) * b; w = c; }
             }
             if (!w) w = 1;
         }
         warps = std::max<uint32_t>(1, std::min<uint32_t>(w, std::min<uint32_t>(16, fit)));
         smem = size_t(warps) * lay.bytes;
-        NBPG_CUDA_TRY(raise_search_attr(device, ops, met, list, false, smem));
+        NBPG_CUDA_TRY(raise_search_attr(device, ops, met, list ? PASS_LIST : PASS_FLAG, false, smem));
         int blocks = 0;
-        NBPG_CUDA_TRY(ops->occ(met, list, false, warps * 32, smem, &blocks));
+        NBPG_CUDA_TRY(ops->occ(met, list ? PASS_LIST : PASS_FLAG, false, warps * 32, smem, &blocks));
         NBPG_CHECK_ARG(blocks >= 1, "search kernel does not fit on an SM");
         grid = uint32_t(blocks) * uint32_t(prop.multiProcessorCount);
         return NBPG_OK;
@@ -231,13 +231,13 @@ extern "C" nbpg_status nbpg_search_noalloc(uint32_t dtype, uint32_t metric, uint
     m.taint = flag_first ? scratch + 4 : nullptr;
     m.lay = lay_main;
     if (plain) {
-        NBPG_CUDA_TRY(raise_search_attr(device, ops, met, !flag_first, true, lay_main.bytes));
-        ops->launch(met, !flag_first, true, nq, 1, lay_main.bytes, m, st);
+        NBPG_CUDA_TRY(raise_search_attr(device, ops, met, flag_first ? PASS_FLAG : PASS_LIST, true, lay_main.bytes));
+        ops->launch(met, flag_first ? PASS_FLAG : PASS_LIST, true, nq, 1, lay_main.bytes, m, st);
     } else {
         uint32_t warps, grid;
         size_t smem;
         if ((s = grid_of(!flag_first, lay_main, P->warps_per_cta, warps, smem, grid)) != NBPG_OK) return s;
-        ops->launch(met, !flag_first, false, grid, warps, smem, m, st);
+        ops->launch(met, flag_first ? PASS_FLAG : PASS_LIST, false, grid, warps, smem, m, st);
     }
     NBPG_CUDA_TRY(cudaGetLastError());
     if (flag_first) {
@@ -249,7 +249,7 @@ extern "C" nbpg_status nbpg_search_noalloc(uint32_t dtype, uint32_t metric, uint
         uint32_t warps, grid;
         size_t smem;
         if ((s = grid_of(true, lay_list, 0, warps, smem, grid)) != NBPG_OK) return s;
-        ops->launch(met, true, false, grid, warps, smem, r, st);
+        ops->launch(met, PASS_LIST, false, grid, warps, smem, r, st);
         NBPG_CUDA_TRY(cudaGetLastError());
     }
     return NBPG_OK;

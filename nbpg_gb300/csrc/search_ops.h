@@ -2,13 +2,15 @@
 // element type compiles in its own translation unit.
 #pragma once
 #include "search_fast.cuh"
+#include "search_flag.cuh"
 
 namespace nbpg {
 
 struct SearchOps {
-    cudaError_t (*set_attr)(int metric, bool list, bool plain, size_t smem);
-    cudaError_t (*occ)(int metric, bool list, bool plain, uint32_t threads, size_t smem, int *blocks);
-    void (*launch)(int metric, bool list, bool plain, uint32_t grid, uint32_t warps, size_t smem, const SearchArgs &a,
+    // pass: a SearchPass (FLAG passes are L2 only: inner product goes straight to LIST)
+    cudaError_t (*set_attr)(int metric, int pass, bool plain, size_t smem);
+    cudaError_t (*occ)(int metric, int pass, bool plain, uint32_t threads, size_t smem, int *blocks);
+    void (*launch)(int metric, int pass, bool plain, uint32_t grid, uint32_t warps, size_t smem, const SearchArgs &a,
                    cudaStream_t st);
     // FAST mode kernels (search_fast.cuh)
     cudaError_t (*set_attr_fast)(int metric, bool plain, size_t smem);
@@ -19,7 +21,7 @@ struct SearchOps {
 
 // Raises a search kernel's dynamic shared-memory attribute to at least smem on `device`, never
 // lowering it (launch plans are cached process-wide and stay valid).
-cudaError_t raise_search_attr(int device, const SearchOps *ops, int metric, bool list, bool plain, size_t smem);
+cudaError_t raise_search_attr(int device, const SearchOps *ops, int metric, int pass, bool plain, size_t smem);
 
 // one table per (element type, uint4 per lane per row)
 #define NBPG_DECL_OPS(t) extern const SearchOps search_ops_##t##_v1, search_ops_##t##_v2, search_ops_##t##_v4;

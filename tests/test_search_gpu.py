@@ -259,3 +259,38 @@ def test_adjacency_word_counter(gpu_lib, mode):
         if mode == "strict":
             r = idx.search(q, qp)
             assert np.array_equal(ids.cpu().numpy().view(np.uint32), r.ids) and np.array_equal(v, r.visited)
+
+
+def _rough_graph(n, R, seed):
+    """Random rows of every degree, some with the same id twice: what a caller may load, and what makes the
+    lossy filter forget and the candidates repeat."""
+    r = np.random.default_rng(seed)
+    g = np.zeros((n, R + 1), np.uint32)
+    g[:, 0] = r.integers(0, R + 1, n)
+    g[0, 0] = R
+    g[:, 1:] = r.integers(0, n, (n, R))
+    if R > 1:
+        g[::7, 2] = g[::7, 1]
+    return g
+
+
+@pytest.mark.parametrize("R", [1, 31, 33, 64, 128])
+@pytest.mark.parametrize("L", [32, 33, 63, 64, 65, 96, 127, 129, 181, 182, 256, 520])
+def test_wide_beams_match_oracle(gpu_lib, oracle_lib, L, R):
+    """Beams around the multiples of 32 (the merge moves 32 positions at a time) and around the filter's
+    sizes, every adjacency chunk count, frontiers that hold every node, cuts that shorten the frontier
+    below a merge's start, repeated start points."""
+    from nbpg_gb300 import synth
+    from nbpg_gb300.index import QueryParams
+    n = 700 if R > 40 else 2500
+    base, q = synth.u8_mixture(n, 24, dim=24, n_centres=6)
+    base[100:140] = base[0:40]  # equal distances
+    g = _rough_graph(n, R, L * 131 + R)
+    idx = _gpu_index(base, g, "u8", "l2")
+    for kernel, cut, k, sp, limit in [("batched", 1.35, 10, (0,), 0), ("plain", 1.0, 5, (0, 0, 9, 9, 9), 0),
+                                      ("batched", 1.05, 1, (3, 140), 37), ("plain", 0.0, 20, (1,), 0)]:
+        if kernel == "plain" and L > 181:
+            kernel = "batched"
+        r = idx.search(q, QueryParams(k=k, beamSize=L, cut=cut, limit=limit), start_points=sp, kernel=kernel)
+        o = oracle_lib.search("u8", "l2", base, g, q, L=L, k=k, cut=cut, limit=limit or None, start_points=sp)
+        _check(r, o, len(q))
