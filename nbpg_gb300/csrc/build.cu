@@ -15,6 +15,7 @@
 #include <vector>
 
 #include "build_impl.cuh"
+#include "build_flag.cuh"
 #include "internal.h"
 
 namespace nbpg {
@@ -81,6 +82,11 @@ static bool kernel_table(uint32_t dtype, uint32_t metric, uint32_t vpl, KernelTa
 }
 
 void row_geometry(uint32_t row_stride, uint32_t want, uint32_t &vecs, uint32_t &lpr, uint32_t &vpl);
+SlotLayout make_flag_layout(uint32_t Lmax, uint32_t R, uint32_t row_stride, bool hash_smem, uint32_t Scap);
+cudaError_t build_flag_search(uint32_t dtype, uint32_t metric, uint32_t grid, uint32_t warps, size_t smem,
+                              const BuildFlagArgs &F, int *blocks, cudaStream_t st);
+cudaError_t build_flag_prune(uint32_t dtype, uint32_t metric, uint32_t grid, const BuildFlagArgs &F, const PruneLayout &lay,
+                             cudaStream_t st);
 
 // dfs.h:46-59
 static bool add_edge_if_possible(std::vector<uint32_t> &G, uint32_t R, size_t from, size_t to)
@@ -192,26 +198,70 @@ static nbpg_status build_impl(nbpg_index *idx, const nbpg_build_params &P, nbpg_
         sa.g_hash_slots = S;
     }
 
+    // The search and prune kernels of build_flag.cuh where their argument holds (VL >= L); a biased candidate
+    // order and FGIM's pair pass stay on the one-kernel insert.
+    bool flag = VL >= L && P.dir_bias_scale <= 0;
+    SlotLayout flay{};
+    PruneLayout play{};
+    uint32_t fw = 0, fgrid = 0;  // warps per CTA, CTAs
+    BuildFlagArgs F{};
+    F.B.s = sa;
+    if (flag) {
+        row_geometry(idx->row_stride, 4, F.B.s.vecs, F.B.s.lpr, F.B.s.vpl);
+        flay = make_flag_layout(L, R, idx->row_stride, !ghash, S);
+        play = make_prune_layout(VL, R, idx->row_stride);
+        flag = flay.bytes <= idx->smem_optin && play.bytes <= idx->smem_optin;
+    }
+    if (flag) {
+        int fb = 0;
+        fw = std::min<uint32_t>(16, uint32_t(idx->smem_optin / flay.bytes));
+        NBPG_CUDA_TRY(build_flag_search(idx->desc.dtype, idx->desc.metric, 0, fw, fw * size_t(flay.bytes), F, &fb, st));
+        NBPG_CUDA_TRY(build_flag_prune(idx->desc.dtype, idx->desc.metric, 0, F, play, st));
+        flag = fb >= 1;
+        fgrid = uint32_t(fb) * uint32_t(idx->sm_count);
+        if (flag && ghash) {
+            if ((s = idx->ghash.ensure(std::max(nslots, size_t(fgrid) * fw) * S * 4)) != NBPG_OK) return s;
+            sa.g_hash = idx->ghash.as<uint32_t>();
+        }
+    }
+
     // batch size (nsw.h:288-295): min(0.02 * n (through float), 1e6), at least 1
     size_t eff = std::min<size_t>(size_t(0.02 * double(float(n))), 1000000ul);
     if (eff == 0) eff = 1;
     const uint32_t nsp_max = std::max<uint32_t>(1, P.num_split);
 
     DevBuf d_inserts, d_sp, d_alpha, d_cos, d_pop, d_sv, d_sd, d_res_ids, d_res_d, d_res_cnt, d_rank, d_cnt, d_off,
-        d_bump, d_grp, d_edges, d_queue, d_bias;
-    ReleaseOnExit release_bufs{{&d_inserts, &d_sp, &d_alpha, &d_cos, &d_pop, &d_sv, &d_sd, &d_res_ids, &d_res_d,
-                                &d_res_cnt, &d_rank, &d_cnt, &d_off, &d_bump, &d_grp, &d_edges, &d_queue, &d_bias}};
+        d_bump, d_grp, d_left, d_edges, d_bias, d_row_d, d_vis, d_near, d_info;
+    ReleaseOnExit release_bufs{{&d_left, &d_row_d, &d_vis, &d_near, &d_info, &d_inserts, &d_sp, &d_alpha, &d_cos, &d_pop, &d_sv, &d_sd, &d_res_ids, &d_res_d,
+                                &d_res_cnt, &d_rank, &d_cnt, &d_off, &d_bump, &d_grp, &d_edges, &d_bias}};
     auto fail_oom = [&](nbpg_status x) { return x; };
     if ((s = d_inserts.ensure(n * 4)) || (s = d_sp.ensure(n * nsp_max * 4)) || (s = d_alpha.ensure(n * 4)) ||
         (s = d_cos.ensure(n * 4)) || (s = d_pop.ensure(n * 4)) || (s = d_sv.ensure(n * 4)) ||
         (s = d_sd.ensure(n * 4)) || (s = d_res_ids.ensure(eff * R * 4)) || (s = d_res_d.ensure(eff * R * 4)) ||
         (s = d_res_cnt.ensure(eff * 4)) || (s = d_rank.ensure(eff * R * 4)) || (s = d_cnt.ensure(n * 4)) ||
-        (s = d_off.ensure(n * 4)) || (s = d_bump.ensure(16)) || (s = d_grp.ensure(eff * R * 4)) ||
-        (s = d_edges.ensure(eff * R * 8)) || (s = d_queue.ensure(16)))
+        (s = d_off.ensure(n * 4)) || (s = d_bump.ensure(32)) || (s = d_grp.ensure(eff * R * 4)) ||
+        (s = d_edges.ensure(eff * R * 8)))
         return fail_oom(s);
     NBPG_CUDA_TRY(cudaMemsetAsync(d_cnt.ptr, 0, n * 4, st));
     NBPG_CUDA_TRY(cudaMemsetAsync(d_sv.ptr, 0, n * 4, st));
     NBPG_CUDA_TRY(cudaMemsetAsync(d_sd.ptr, 0, n * 4, st));
+
+    // The neighbours' distances beside the graph, for rev_insert_kernel.  With top_degree the merge
+    // orders by interpolated distances: then, and where this does not fit, every target takes the
+    // general merge.
+    bool keep_d = P.top_degree == 0 || P.top_degree == R;
+    if (keep_d && ((s = d_left.ensure(eff * R * 4)) || (s = d_row_d.ensure(size_t(n) * R * 4)))) {
+        cudaGetLastError();
+        keep_d = false;
+    }
+
+    if (flag) {
+        if ((s = d_vis.ensure(eff * FLAG_VIS * 8)) || (s = d_near.ensure(eff * R * 8)) || (s = d_info.ensure(eff * 16)))
+            return fail_oom(s);
+        F.vis = d_vis.as<uint64_t>();
+        F.near = d_near.as<uint64_t>();
+        F.info = d_info.as<uint4>();
+    }
 
     BuildArgs B{};
     B.s = sa;
@@ -230,6 +280,12 @@ static nbpg_status build_impl(nbpg_index *idx, const nbpg_build_params &P, nbpg_
     B.bump = d_bump.as<uint32_t>();
     B.grp_target = d_grp.as<uint32_t>();
     B.edges = d_edges.as<uint64_t>();
+    if (keep_d) {
+        B.row_d = d_row_d.as<float>();
+        B.grp_left = d_left.as<uint32_t>();
+        rows_unknown_kernel<<<uint32_t((n + 255) / 256), 256, 0, st>>>(B);
+        NBPG_CUDA_TRY(cudaGetLastError());
+    }
     B.dir_bias = nullptr;
     std::vector<double> bias_host;
     if (P.dir_bias_scale > 0) {
@@ -315,11 +371,21 @@ static nbpg_status build_impl(nbpg_index *idx, const nbpg_build_params &P, nbpg_
             B.inserts = d_inserts.as<uint32_t>() + lo;
             B.sp = d_sp.as<uint32_t>() + lo * nsp;
             B.bs = bs;
-            B.queue = d_queue.as<uint32_t>();
-            NBPG_CUDA_TRY(cudaMemsetAsync(d_queue.ptr, 0, 16, st));
-            NBPG_CUDA_TRY(cudaMemsetAsync(d_bump.ptr, 0, 16, st));
+            B.queue = B.bump + 4;  // bump: edge allocator, groups, groups left; from 4 the work counters
+            NBPG_CUDA_TRY(cudaMemsetAsync(d_bump.ptr, 0, 32, st));
             const uint32_t g1 = std::min<uint32_t>(full_grid, (bs + W - 1) / W);
-            kt.search(g1, W * 32, smem_search, B, st);
+            if (flag && !pair) {
+                const SearchArgs geometry = F.B.s;  // this kernel's lanes per row
+                F.B = B;
+                F.B.s.lpr = geometry.lpr;
+                F.B.s.vpl = geometry.vpl;
+                F.B.s.lay = flay;
+                const uint32_t gf = std::min<uint32_t>(fgrid, (bs + fw - 1) / fw);
+                NBPG_CUDA_TRY(build_flag_search(idx->desc.dtype, idx->desc.metric, gf, fw, fw * size_t(flay.bytes), F, nullptr, st));
+                NBPG_CUDA_TRY(build_flag_prune(idx->desc.dtype, idx->desc.metric, bs, F, play, st));
+            } else {
+                kt.search(g1, W * 32, smem_search, B, st);
+            }
             BuildArgs Wr = B;
             Wr.s.graph = wg;
             forward_write_kernel<<<bs, 64, 0, st>>>(Wr);
@@ -329,7 +395,13 @@ static nbpg_status build_impl(nbpg_index *idx, const nbpg_build_params &P, nbpg_
             rev_alloc_kernel<<<eg, 256, 0, st>>>(B);
             rev_scatter_kernel<<<eg, 256, 0, st>>>(B);
             BuildArgs M = Wr;
-            M.queue = d_queue.as<uint32_t>() + 1;
+            M.queue = B.bump + 5;
+            if (keep_d) {
+                const uint32_t gi = std::min<uint32_t>(uint32_t(idx->sm_count) * 8, (ne + 7) / 8);
+                if (R <= 32) rev_insert_kernel<1><<<gi, 256, 0, st>>>(M);
+                else if (R <= 64) rev_insert_kernel<2><<<gi, 256, 0, st>>>(M);
+                else rev_insert_kernel<4><<<gi, 256, 0, st>>>(M);
+            }
             const uint32_t gm = std::min<uint32_t>(uint32_t(idx->sm_count) * 8, (ne + MW - 1) / MW);
             kt.merge(gm, MW * 32, smem_merge, M, st);
             NBPG_CUDA_TRY(cudaGetLastError());
@@ -436,9 +508,6 @@ static nbpg_status build_impl(nbpg_index *idx, const nbpg_build_params &P, nbpg_
     if (out_sv) NBPG_CUDA_TRY(cudaMemcpyAsync(out_sv, d_sv.ptr, n * 4, cudaMemcpyDeviceToHost, st));
     if (out_sd) NBPG_CUDA_TRY(cudaMemcpyAsync(out_sd, d_sd.ptr, n * 4, cudaMemcpyDeviceToHost, st));
     NBPG_CUDA_TRY(cudaStreamSynchronize(st));
-    for (DevBuf *b : {&d_inserts, &d_sp, &d_alpha, &d_cos, &d_pop, &d_sv, &d_sd, &d_res_ids, &d_res_d, &d_res_cnt,
-                      &d_rank, &d_cnt, &d_off, &d_bump, &d_grp, &d_edges, &d_queue, &d_bias})
-        b->release();
     if (stats) {
         stats->isolated = iso;
         stats->batches = batches;

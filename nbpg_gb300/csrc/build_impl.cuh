@@ -13,7 +13,10 @@
 //      contiguous block, edges scatter into it (merge_edges.h:53-81 up to order).
 //   6. rev_merge_kernel           one warp per target: the VL smallest (dist, source)
 //      reverse edges (merge_edges.h:98-119), plus existing neighbours not repeated,
-//      new distances, sort or truncate to R (nsw.h:463-511, 329-378).
+//      new distances, sort or truncate to R (nsw.h:463-511, 329-378).  The flat build keeps
+//      the neighbours' distances beside the graph (row_d), so that most targets, with a few
+//      new edges and a sorted row, take rev_insert_kernel instead: two sorted lists merged
+//      by counting, without reading a vector.
 #pragma once
 #include "search_impl.cuh"
 
@@ -43,6 +46,8 @@ struct BuildArgs {
     uint32_t *bump;        // [0] allocator, [1] group count
     uint32_t *grp_target;  // groups
     uint64_t *edges;       // grouped (dist, source) keys
+    float *row_d;          // [n][R] distances of the rows' neighbours, NaN first where unknown; or null
+    uint32_t *grp_left;    // targets rev_insert_kernel leaves to rev_merge_kernel; count in bump[2]
     uint32_t pair;         // FGIM pair pass (FGIM_nsw.h:45-109) instead of searchNghAndPrune
     const double *dir_bias;  // sort_candidates' degree bias: factor per degree d in [0, R],
                              // dir_bias_scale * log(d + 1) + 1 (prune.h:59-63); null = none
@@ -449,6 +454,16 @@ static __global__ void forward_write_kernel(BuildArgs B)
     uint32_t *row = const_cast<uint32_t *>(B.s.graph) + size_t(index) * B.s.gstride;
     for (uint32_t j = threadIdx.x; j <= B.R; j += blockDim.x)
         row[j] = j == 0 ? cnt : (j - 1 < cnt ? B.res_ids[size_t(t) * B.R + j - 1] : 0u);
+    if (B.row_d)
+        for (uint32_t j = threadIdx.x; j < cnt; j += blockDim.x)
+            B.row_d[size_t(index) * B.R + j] = B.res_d[size_t(t) * B.R + j];
+}
+
+// Rows that already have neighbours (a graph given before the build): their distances are unknown.
+static __global__ void rows_unknown_kernel(BuildArgs B)
+{
+    const size_t v = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (v < B.s.n && B.s.graph[v * B.s.gstride]) B.row_d[v * B.R] = __int_as_float(0x7fc00000);
 }
 
 static __global__ void rev_count_kernel(BuildArgs B)
@@ -460,15 +475,51 @@ static __global__ void rev_count_kernel(BuildArgs B)
     B.rank[e] = atomicAdd(&B.cnt_node[B.res_ids[e]], 1u);
 }
 
-static __global__ void rev_alloc_kernel(BuildArgs B)
+// Blocks of 256 threads.  The two counters are taken once per block: one atomic per edge on the same
+// two words took 20 us of a 2,000-insert batch.
+static __global__ void __launch_bounds__(256) rev_alloc_kernel(BuildArgs B)
 {
+    __shared__ uint32_t wsum[8], wcnt[8], base[2];
     const size_t e = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (e >= size_t(B.bs) * B.R) return;
-    const uint32_t t = uint32_t(e / B.R), j = uint32_t(e % B.R);
-    if (j >= B.res_cnt[t] || B.rank[e] != 0) return;
-    const uint32_t target = B.res_ids[e];
-    B.off_node[target] = atomicAdd(&B.bump[0], B.cnt_node[target]);
-    B.grp_target[atomicAdd(&B.bump[1], 1u)] = target;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    bool first = false;
+    uint32_t target = 0, edges = 0;
+    if (e < size_t(B.bs) * B.R) {
+        const uint32_t t = uint32_t(e / B.R), j = uint32_t(e % B.R);
+        first = j < B.res_cnt[t] && B.rank[e] == 0;
+        if (first) {
+            target = B.res_ids[e];
+            edges = B.cnt_node[target];
+        }
+    }
+    const unsigned m = __ballot_sync(kFull, first);
+    uint32_t incl = edges;
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t x = __shfl_up_sync(kFull, incl, o);
+        if (lane >= o) incl += x;
+    }
+    if (lane == 31) {
+        wsum[warp] = incl;
+        wcnt[warp] = __popc(m);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        uint32_t s = 0, c = 0;
+        for (int w = 0; w < 8; ++w) {
+            const uint32_t ws = wsum[w], wc = wcnt[w];
+            wsum[w] = s;
+            wcnt[w] = c;
+            s += ws;
+            c += wc;
+        }
+        base[0] = s ? atomicAdd(&B.bump[0], s) : 0u;
+        base[1] = c ? atomicAdd(&B.bump[1], c) : 0u;
+    }
+    __syncthreads();
+    if (first) {
+        B.off_node[target] = base[0] + wsum[warp] + incl - edges;
+        B.grp_target[base[1] + wcnt[warp] + __popc(m & lanemask_lt())] = target;
+    }
 }
 
 static __global__ void rev_scatter_kernel(BuildArgs B)
@@ -479,6 +530,93 @@ static __global__ void rev_scatter_kernel(BuildArgs B)
     if (j >= B.res_cnt[t]) return;
     const uint32_t target = B.res_ids[e];
     B.edges[B.off_node[target] + B.rank[e]] = make_key(B.res_d[e], B.inserts[t]);
+}
+
+// One warp per target, RC = ceil(R / 32) row entries per lane: at most 32 new edges go into a row
+// whose distances are known and in order.  An existing neighbour that is also a new source is dropped
+// (nsw.h:358-378: the new entry stands first); every entry's place is its index plus the number of
+// entries of the other list before it.  Every other target goes on to rev_merge_kernel.
+// Bound by latency of scattered reads, about 1 KB per target in place of the 7 KB that reading every
+// neighbour's vector takes.
+template <int RC>
+__global__ void __launch_bounds__(256) rev_insert_kernel(BuildArgs B)
+{
+    const int lane = threadIdx.x & 31;
+    const uint32_t R = B.R, ngroups = B.bump[1], warps = gridDim.x * (blockDim.x >> 5);
+    for (uint32_t g = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); g < ngroups; g += warps) {
+        const uint32_t target = B.grp_target[g];
+        const uint32_t size = B.cnt_node[target];
+        uint32_t *row = const_cast<uint32_t *>(B.s.graph) + size_t(target) * B.s.gstride;
+        float *rd = B.row_d + size_t(target) * R;
+        const uint32_t deg = row[0];
+        uint64_t key[RC];
+        bool odd = size > 32 || size > B.VL;  // not for this kernel
+#pragma unroll
+        for (int c = 0; c < RC; ++c) {
+            const uint32_t i = c * 32 + lane;
+            key[c] = kKeyMax;
+            if (i < deg) {
+                const float d = rd[i];
+                odd |= d != d;
+                key[c] = make_key(d, row[1 + i]);
+            }
+        }
+        const uint64_t e = !odd && uint32_t(lane) < size ? B.edges[B.off_node[target] + lane] : kKeyMax;
+#pragma unroll
+        for (int c = 0; c < RC; ++c) {
+            const uint64_t head = c + 1 < RC ? __shfl_sync(kFull, key[c + 1 < RC ? c + 1 : c], 0) : kKeyMax;
+            uint64_t next = __shfl_down_sync(kFull, key[c], 1);
+            if (lane == 31) next = head;
+            odd |= key[c] > next;
+        }
+        if (__any_sync(kFull, odd)) {
+            if (lane == 0) B.grp_left[atomicAdd(&B.bump[2], 1u)] = target;
+            continue;
+        }
+        bool keep[RC];
+        uint32_t at[RC];  // entry's place
+        unsigned kept[RC];
+#pragma unroll
+        for (int c = 0; c < RC; ++c) keep[c] = c * 32 + lane < int(deg);
+        for (uint32_t j = 0; j < size; ++j) {
+            const uint32_t src = key_id(__shfl_sync(kFull, e, int(j)));
+#pragma unroll
+            for (int c = 0; c < RC; ++c) keep[c] = keep[c] && key_id(key[c]) != src;
+        }
+        uint32_t nk = 0;
+#pragma unroll
+        for (int c = 0; c < RC; ++c) {
+            kept[c] = __ballot_sync(kFull, keep[c]);
+            at[c] = nk + __popc(kept[c] & lanemask_lt());
+            nk += __popc(kept[c]);
+        }
+        uint32_t mine = 0;  // this lane's new edge's place
+        for (uint32_t j = 0; j < size; ++j) {
+            const uint64_t ej = __shfl_sync(kFull, e, int(j));
+            uint32_t below = __popc(__ballot_sync(kFull, e < ej));
+#pragma unroll
+            for (int c = 0; c < RC; ++c) {
+                below += __popc(__ballot_sync(kFull, keep[c] && key[c] < ej));
+                at[c] += ej < key[c];
+            }
+            if (uint32_t(lane) == j) mine = below;
+        }
+#pragma unroll
+        for (int c = 0; c < RC; ++c)
+            if (keep[c] && at[c] < R) {
+                row[1 + at[c]] = key_id(key[c]);
+                rd[at[c]] = key_dist(key[c]);
+            }
+        if (uint32_t(lane) < size && mine < R) {
+            row[1 + mine] = key_id(e);
+            rd[mine] = key_dist(e);
+        }
+        if (lane == 0) {
+            row[0] = min(size + nk, R);  // at least deg: the slots past it are zero already
+            if (B.stat_dist) B.stat_dist[target] += nk;  // the reference computes the kept neighbours' distances
+            B.cnt_node[target] = 0;
+        }
+    }
 }
 
 // per-warp shared memory of rev_merge_kernel
@@ -496,13 +634,13 @@ __global__ void __launch_bounds__(256) rev_merge_kernel(BuildArgs B)
     uint64_t *cand = reinterpret_cast<uint64_t *>(ws);
     uint32_t *ids = reinterpret_cast<uint32_t *>(ws + kMergeCap * 8);
     uint64_t *exact = reinterpret_cast<uint64_t *>(ws + kMergeCap * 8 + 128 * 4);
-    const uint32_t ngroups = B.bump[1];
+    const uint32_t ngroups = B.grp_left ? B.bump[2] : B.bump[1];
     while (true) {
         uint32_t g = 0;
         if (lane == 0) g = atomicAdd(B.queue, 1u);
         g = __shfl_sync(kFull, g, 0);
         if (g >= ngroups) break;
-        const uint32_t target = B.grp_target[g];
+        const uint32_t target = B.grp_left ? B.grp_left[g] : B.grp_target[g];
         const uint32_t size = B.cnt_node[target];
         const uint64_t *E = B.edges + B.off_node[target];
 
@@ -587,6 +725,8 @@ __global__ void __launch_bounds__(256) rev_merge_kernel(BuildArgs B)
         uint32_t *row = const_cast<uint32_t *>(a.graph) + size_t(target) * a.gstride;
         for (uint32_t j = lane; j <= R; j += 32)
             row[j] = j == 0 ? outn : (j - 1 < outn ? key_id(cand[j - 1]) : 0u);
+        if (B.row_d)
+            for (uint32_t j = lane; j < outn; j += 32) B.row_d[size_t(target) * R + j] = key_dist(cand[j]);
         if (lane == 0) {
             if (B.stat_dist) B.stat_dist[target] += rp;
             B.cnt_node[target] = 0;

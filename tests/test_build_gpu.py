@@ -123,3 +123,49 @@ def test_fgim_dir_bias_matches_oracle(gpu_lib, oracle_lib, dtype, metric):
     assert np.array_equal(_mask(idx.get_graph()), _mask(go))
     assert st.isolated == iso
     assert np.array_equal(gsv, sv) and np.array_equal(gsd, sd)
+
+
+@pytest.mark.parametrize("dtype,metric,n,dims,R,L,VL,split,passes,dyn", [
+    ("u8", "l2", 900, 32, 16, 24, 24, 0, 1, False),      # VL = L
+    ("u8", "l2", 900, 32, 16, 33, 32, 0, 2, False),      # VL < L: the one-kernel insert
+    ("i8", "ip", 1500, 100, 32, 64, 96, 0, 2, True),     # odd rows, inner product
+    ("u8", "l2", 1500, 16, 64, 100, 192, 4, 2, True),    # VL + R = 256
+    ("u8", "l2", 1200, 48, 128, 110, 128, 0, 2, False),  # four adjacency chunks
+    ("u8", "l2", 1200, 400, 24, 40, 160, 0, 1, False),   # the candidates' rows do not fit: read from memory
+    ("u4", "l2", 2000, 33, 33, 65, 80, 2, 2, True),      # three-word rows, degree past one chunk
+    ("u8", "l2", 700, 24, 1, 2, 255, 0, 1, False),       # a single edge per node
+    ("u8", "l2", 40, 24, 8, 200, 248, 0, 1, False),      # fewer rows than the beam
+    ("u8", "l2", 1800, 24, 16, 190, 230, 0, 1, False),   # filter in global memory
+])
+def test_build_kernel_edges(gpu_lib, oracle_lib, dtype, metric, n, dims, R, L, VL, split, passes, dyn):
+    """The search / prune kernels and the reverse-edge insert at the edges of their ranges: graphs and
+    counters equal the oracle's."""
+    from nbpg_gb300.index import Index
+    base = _data(dtype, n=n, dims=dims)
+    base[n // 2:n // 2 + 10] = base[:10]  # equal rows
+    kw = dict(L=L, VL=VL, num_split=split, num_passes=passes, dynamic_prune=dyn, min_alpha=1.05 if dyn else 1.0,
+              max_alpha=1.2, sp_seed=5)
+    go, sv, sd, iso = oracle_lib.build_graph(dtype, metric, base, R=R, **kw)
+    idx = Index(base, dtype, metric, max_degree=R)
+    st, gsv, gsd = idx.build_vamana(**kw, with_stats=True)
+    assert np.array_equal(_mask(idx.get_graph()), _mask(go))
+    assert st.isolated == iso and np.array_equal(gsv, sv) and np.array_equal(gsd, sd)
+
+
+def test_build_over_unsorted_rows(gpu_lib, oracle_lib):
+    """A prior graph whose rows are in no order and hold an id twice: their distances are unknown to the
+    reverse-edge insert, and the merge's neighbour order and repeats are the reference's."""
+    from nbpg_gb300.index import Index
+    base = _data("u8", n=1500)
+    r = np.random.default_rng(3)
+    g0 = np.zeros((1500, 17), np.uint32)
+    g0[:, 0] = r.integers(0, 17, 1500)
+    g0[:, 1:] = r.integers(0, 1500, (1500, 16))
+    g0[::5, 2] = g0[::5, 1]
+    g0[:, 1:][np.arange(16)[None, :] >= g0[:, :1]] = 0
+    kw = dict(L=24, VL=32, num_split=0, num_passes=2, max_alpha=1.2)
+    go, sv, sd, _ = oracle_lib.build_graph("u8", "l2", base, R=16, graph=g0, **kw)
+    idx = Index(base, "u8", "l2", max_degree=16, graph=g0)
+    _, gsv, gsd = idx.build_vamana(**kw, with_stats=True)
+    assert np.array_equal(_mask(idx.get_graph()), _mask(go))
+    assert np.array_equal(gsv, sv) and np.array_equal(gsd, sd)
