@@ -10,8 +10,8 @@
 #include <chrono>
 #include <cmath>
 #include <numeric>
-#include <queue>
 #include <random>
+#include <unordered_map>
 #include <vector>
 
 #include "build_impl.cuh"
@@ -88,47 +88,214 @@ cudaError_t build_flag_search(uint32_t dtype, uint32_t metric, uint32_t grid, ui
 cudaError_t build_flag_prune(uint32_t dtype, uint32_t metric, uint32_t grid, const BuildFlagArgs &F, const PruneLayout &lay,
                              cudaStream_t st);
 
-// dfs.h:46-59
-static bool add_edge_if_possible(std::vector<uint32_t> &G, uint32_t R, size_t from, size_t to)
+// ---------------------------------------------------------------------------
+// Isolated-node repair (dfs.h:63-137, 193-215).  Reachability from the entry is a breadth-first sweep on
+// the device (which nodes are reached does not depend on the order); the repair itself depends on the order
+// of the nodes, so it runs on the host, over copies of the few rows it can touch.  Copying the whole graph
+// to the host and walking it there took 24 ms of a 61 ms build at 100k rows, 52 of 277 ms at 250k.
+// ---------------------------------------------------------------------------
+constexpr uint32_t REACH_LEVELS = 16;  // levels per round of launches
+constexpr uint32_t REACH_MOST = 256;   // deeper graphs (long chains of one edge per node) are walked on the host
+
+// One level: a warp per node of [head[level], head[level + 1]) of the queue marks its neighbours and appends
+// the new ones.  `head` holds the queue's end after every level (head[0] = 0, head[1] = 1: the entry).
+static __global__ void __launch_bounds__(256) reach_level_kernel(const uint32_t *graph, uint32_t gstride, uint32_t *seen,
+                                                                 uint32_t *queue, uint32_t *head, uint32_t level)
 {
-    uint32_t *r = &G[from * (R + 1)];
+    const uint32_t lane = threadIdx.x & 31, from = head[level], to = head[level + 1];
+    for (uint32_t i = from + blockIdx.x * 8 + (threadIdx.x >> 5); i < to; i += gridDim.x * 8) {
+        const uint32_t *row = graph + size_t(queue[i]) * gstride;
+        const uint32_t deg = row[0];
+        for (uint32_t j = 0; j < deg; j += 32) {
+            const uint32_t v = j + lane < deg ? row[1 + j + lane] : 0u;
+            const bool fresh = j + lane < deg && !((seen[v >> 5] >> (v & 31)) & 1) &&
+                               !((atomicOr(&seen[v >> 5], 1u << (v & 31)) >> (v & 31)) & 1);
+            const unsigned m = __ballot_sync(kFull, fresh);
+            uint32_t at = 0;
+            if (m && lane == 0) at = atomicAdd(&head[level + 2], uint32_t(__popc(m)));
+            at = __shfl_sync(kFull, at, 0);
+            // head[level + 2] counts this level's new nodes from zero; they follow those before
+            if (fresh) queue[to + at + __popc(m & lanemask_lt())] = v;
+        }
+    }
+}
+
+// Turns the count of the level just run into the queue's end (one thread, after the level's kernel)
+static __global__ void reach_close_kernel(uint32_t *head, uint32_t level) { head[level + 2] += head[level + 1]; }
+
+static __global__ void reach_start_kernel(uint32_t *seen, uint32_t *queue, uint32_t *head, uint32_t entry)
+{
+    queue[0] = entry;
+    head[1] = 1;
+    seen[entry >> 5] = 1u << (entry & 31);
+}
+
+static __global__ void rows_gather_kernel(const uint32_t *graph, uint32_t gstride, uint32_t words, const uint32_t *ids,
+                                          uint32_t *out)
+{
+    for (uint32_t j = threadIdx.x; j < words; j += blockDim.x)
+        out[size_t(blockIdx.x) * words + j] = graph[size_t(ids[blockIdx.x]) * gstride + j];
+}
+
+static __global__ void rows_scatter_kernel(uint32_t *graph, uint32_t gstride, uint32_t words, const uint32_t *ids,
+                                           const uint32_t *in)
+{
+    for (uint32_t j = threadIdx.x; j < words; j += blockDim.x)
+        graph[size_t(ids[blockIdx.x]) * gstride + j] = in[size_t(blockIdx.x) * words + j];
+}
+
+// Host copies of graph rows, fetched when first asked for and written back together
+struct RowCache {
+    nbpg_index *idx;
+    std::unordered_map<uint32_t, uint32_t> at;  // node -> row in `rows`
+    std::vector<uint32_t> ids, rows;
+    DevBuf d_ids, d_rows;
+    ReleaseOnExit release{{&d_ids, &d_rows}};
+    uint32_t words() const { return idx->desc.max_degree + 1; }
+    nbpg_status fetch(const std::vector<uint32_t> &want)
+    {
+        std::vector<uint32_t> miss;
+        for (uint32_t v : want)
+            if (at.emplace(v, uint32_t(ids.size() + miss.size())).second) miss.push_back(v);
+        if (miss.empty()) return NBPG_OK;
+        nbpg_status s;
+        const size_t bytes = miss.size() * words() * 4;
+        if ((s = d_ids.ensure(miss.size() * 4)) || (s = d_rows.ensure(bytes))) return s;
+        NBPG_CUDA_TRY(cudaMemcpyAsync(d_ids.ptr, miss.data(), miss.size() * 4, cudaMemcpyHostToDevice, idx->stream));
+        rows_gather_kernel<<<uint32_t(miss.size()), 64, 0, idx->stream>>>(idx->d_graph, idx->gstride, words(),
+                                                                          d_ids.as<uint32_t>(), d_rows.as<uint32_t>());
+        NBPG_CUDA_TRY(cudaGetLastError());
+        const size_t old = rows.size();
+        rows.resize(old + miss.size() * words());
+        NBPG_CUDA_TRY(cudaMemcpyAsync(rows.data() + old, d_rows.ptr, bytes, cudaMemcpyDeviceToHost, idx->stream));
+        NBPG_CUDA_TRY(cudaStreamSynchronize(idx->stream));
+        ids.insert(ids.end(), miss.begin(), miss.end());
+        return NBPG_OK;
+    }
+    uint32_t *row(uint32_t v) { return &rows[size_t(at.at(v)) * words()]; }
+    nbpg_status write_back()
+    {
+        if (ids.empty()) return NBPG_OK;
+        nbpg_status s;
+        if ((s = d_ids.ensure(ids.size() * 4)) || (s = d_rows.ensure(rows.size() * 4))) return s;
+        NBPG_CUDA_TRY(cudaMemcpyAsync(d_ids.ptr, ids.data(), ids.size() * 4, cudaMemcpyHostToDevice, idx->stream));
+        NBPG_CUDA_TRY(cudaMemcpyAsync(d_rows.ptr, rows.data(), rows.size() * 4, cudaMemcpyHostToDevice, idx->stream));
+        rows_scatter_kernel<<<uint32_t(ids.size()), 64, 0, idx->stream>>>(idx->d_graph, idx->gstride, words(),
+                                                                          d_ids.as<uint32_t>(), d_rows.as<uint32_t>());
+        NBPG_CUDA_TRY(cudaGetLastError());
+        NBPG_CUDA_TRY(cudaStreamSynchronize(idx->stream));
+        return NBPG_OK;
+    }
+};
+
+// dfs.h:46-59
+static bool add_edge_if_possible(uint32_t *r, uint32_t R, uint32_t to)
+{
     if (r[0] >= R) return false;
     for (uint32_t k = 0; k < r[0]; ++k)
         if (r[1 + k] == to) return true;
-    r[1 + r[0]] = uint32_t(to);
+    r[1 + r[0]] = to;
     r[0] += 1;
     return true;
 }
 
-// dfs.h:63-137, 193-215: BFS from the entry, then give every unreachable node an in-edge.
-static size_t repair_isolated(std::vector<uint32_t> &G, uint32_t R, uint64_t n, uint32_t entry)
+// Every node unreachable from the entry gets an in-edge; *count receives how many there were.
+static nbpg_status repair_isolated(nbpg_index *idx, uint32_t entry, uint64_t *count)
 {
-    std::vector<int> flag(n, 0);
-    std::queue<size_t> q;
-    flag[entry] = 1;
-    q.push(entry);
-    while (!q.empty()) {
-        size_t v = q.front();
-        q.pop();
-        const uint32_t *r = &G[v * (R + 1)];
-        for (uint32_t j = 0; j < r[0]; ++j)
-            if (!flag[r[1 + j]]) { flag[r[1 + j]] = 1; q.push(r[1 + j]); }
+    const uint32_t R = idx->desc.max_degree, n = uint32_t(idx->desc.n);
+    const size_t words = (size_t(n) + 31) / 32;
+    cudaStream_t st = idx->stream;
+    DevBuf d_seen, d_queue, d_head;
+    ReleaseOnExit release{{&d_seen, &d_queue, &d_head}};
+    nbpg_status s;
+    const size_t heads = REACH_MOST + 2;
+    if ((s = d_seen.ensure(words * 4)) || (s = d_queue.ensure(size_t(n) * 4)) || (s = d_head.ensure(heads * 4))) return s;
+    NBPG_CUDA_TRY(cudaMemsetAsync(d_seen.ptr, 0, words * 4, st));
+    NBPG_CUDA_TRY(cudaMemsetAsync(d_head.ptr, 0, heads * 4, st));
+    uint32_t *head = d_head.as<uint32_t>();
+    reach_start_kernel<<<1, 1, 0, st>>>(d_seen.as<uint32_t>(), d_queue.as<uint32_t>(), head, entry);
+    const uint32_t grid = uint32_t(std::min<size_t>(size_t(idx->sm_count) * 8, size_t(n) / 8 + 1));
+    bool swept = false;
+    for (uint32_t level = 0; level < REACH_MOST && !swept; ++level) {
+        reach_level_kernel<<<grid, 256, 0, st>>>(idx->d_graph, idx->gstride, d_seen.as<uint32_t>(), d_queue.as<uint32_t>(),
+                                                 head, level);
+        reach_close_kernel<<<1, 1, 0, st>>>(head, level);
+        NBPG_CUDA_TRY(cudaGetLastError());
+        if ((level + 1) % REACH_LEVELS == 0) {
+            uint32_t h[2];
+            NBPG_CUDA_TRY(cudaMemcpyAsync(h, head + level + 1, 8, cudaMemcpyDeviceToHost, st));
+            NBPG_CUDA_TRY(cudaStreamSynchronize(st));
+            swept = h[0] == h[1];  // the last level found nothing new
+        }
     }
-    size_t cnt = 0;
-    for (size_t i = 0; i < n; ++i) {
-        if (flag[i]) continue;
-        ++cnt;
-        const uint32_t *r = &G[i * (R + 1)];
+    std::vector<uint32_t> seen(words, 0u);
+    if (swept) {
+        NBPG_CUDA_TRY(cudaMemcpyAsync(seen.data(), d_seen.ptr, words * 4, cudaMemcpyDeviceToHost, st));
+        NBPG_CUDA_TRY(cudaStreamSynchronize(st));
+    } else {
+        std::vector<uint32_t> G(size_t(n) * (R + 1)), queue{entry};
+        NBPG_CUDA_TRY(cudaMemcpy2DAsync(G.data(), (R + 1) * 4, idx->d_graph, idx->gstride * 4, (R + 1) * 4, n,
+                                        cudaMemcpyDeviceToHost, st));
+        NBPG_CUDA_TRY(cudaStreamSynchronize(st));
+        seen[entry >> 5] |= 1u << (entry & 31);
+        for (size_t h = 0; h < queue.size(); ++h) {
+            const uint32_t *r = &G[size_t(queue[h]) * (R + 1)];
+            for (uint32_t j = 0; j < r[0]; ++j) {
+                const uint32_t v = r[1 + j], bit = 1u << (v & 31);
+                if (!(seen[v >> 5] & bit)) {
+                    seen[v >> 5] |= bit;
+                    queue.push_back(v);
+                }
+            }
+        }
+    }
+    auto reached = [&](uint32_t v) { return ((seen[v >> 5] >> (v & 31)) & 1) != 0; };
+    std::vector<uint32_t> lost;
+    for (uint32_t w = 0; w < words; ++w) {
+        uint32_t m = ~seen[w];
+        if (size_t(w) * 32 + 32 > n) m &= (1u << (n & 31)) - 1u;
+        for (; m; m &= m - 1) lost.push_back(w * 32 + uint32_t(__builtin_ctz(m)));
+    }
+    *count = lost.size();
+    if (lost.empty()) return NBPG_OK;
+    // the rows the repair reads and writes: the lost nodes', their neighbours' and the entry's
+    RowCache rc{idx, {}, {}, {}, {}, {}};
+    std::vector<uint32_t> want(lost);
+    want.push_back(entry);
+    if ((s = rc.fetch(want)) != NBPG_OK) return s;
+    want.clear();
+    for (uint32_t i : lost) {
+        const uint32_t *r = rc.row(i);
+        want.insert(want.end(), r + 1, r + 1 + r[0]);
+    }
+    if ((s = rc.fetch(want)) != NBPG_OK) return s;
+    for (uint32_t i : lost) {
+        // a neighbour list of its own: adding an edge below can lengthen this node's row while it is walked
+        // only by the node itself, which add_edge_if_possible refuses to repeat
         bool done = false;
-        for (uint32_t j = 0; j < r[0] && !done; ++j)
-            if (flag[r[1 + j]] == 1 && add_edge_if_possible(G, R, r[1 + j], i)) done = true;
-        for (uint32_t j = 0; j < r[0] && !done; ++j)
-            if (add_edge_if_possible(G, R, r[1 + j], i)) done = true;
-        if (!done && flag[entry] == 1 && add_edge_if_possible(G, R, entry, i)) done = true;
-        for (size_t x = 0; x < n && !done; ++x)
-            if (flag[x] == 1 && add_edge_if_possible(G, R, x, i)) done = true;
+        for (uint32_t j = 0; j < rc.row(i)[0] && !done; ++j) {
+            const uint32_t v = rc.row(i)[1 + j];
+            if (reached(v)) done = add_edge_if_possible(rc.row(v), R, i);
+        }
+        for (uint32_t j = 0; j < rc.row(i)[0] && !done; ++j) {
+            const uint32_t v = rc.row(i)[1 + j];
+            if (rc.at.find(v) == rc.at.end() && (s = rc.fetch({v})) != NBPG_OK) return s;
+            done = add_edge_if_possible(rc.row(v), R, i);
+        }
+        if (!done) done = add_edge_if_possible(rc.row(entry), R, i);
+        for (uint32_t x = 0; x < n && !done; ++x) {
+            if (!reached(x)) continue;
+            if (rc.at.find(x) == rc.at.end()) {
+                // the nodes from here on, a thousand at a time
+                std::vector<uint32_t> next;
+                for (uint32_t y = x; y < n && next.size() < 1024; ++y)
+                    if (reached(y)) next.push_back(y);
+                if ((s = rc.fetch(next)) != NBPG_OK) return s;
+            }
+            done = add_edge_if_possible(rc.row(x), R, i);
+        }
     }
-    return cnt;
+    return rc.write_back();
 }
 
 struct DevArr {
@@ -496,14 +663,7 @@ static nbpg_status build_impl(nbpg_index *idx, const nbpg_build_params &P, nbpg_
 
     uint64_t iso = 0;
     if (P.repair_isolate) {
-        std::vector<uint32_t> G(size_t(n) * (R + 1));
-        NBPG_CUDA_TRY(cudaMemcpy2DAsync(G.data(), (R + 1) * 4, idx->d_graph, idx->gstride * 4, (R + 1) * 4, n,
-                                        cudaMemcpyDeviceToHost, st));
-        NBPG_CUDA_TRY(cudaStreamSynchronize(st));
-        iso = repair_isolated(G, R, n, 0);
-        if (iso)
-            NBPG_CUDA_TRY(cudaMemcpy2DAsync(idx->d_graph, idx->gstride * 4, G.data(), (R + 1) * 4, (R + 1) * 4, n,
-                                            cudaMemcpyHostToDevice, st));
+        if ((s = repair_isolated(idx, 0, &iso)) != NBPG_OK) return s;
     }
     if (out_sv) NBPG_CUDA_TRY(cudaMemcpyAsync(out_sv, d_sv.ptr, n * 4, cudaMemcpyDeviceToHost, st));
     if (out_sd) NBPG_CUDA_TRY(cudaMemcpyAsync(out_sd, d_sd.ptr, n * 4, cudaMemcpyDeviceToHost, st));
