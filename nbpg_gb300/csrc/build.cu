@@ -82,7 +82,7 @@ static bool kernel_table(uint32_t dtype, uint32_t metric, uint32_t vpl, KernelTa
 }
 
 void row_geometry(uint32_t row_stride, uint32_t want, uint32_t &vecs, uint32_t &lpr, uint32_t &vpl);
-SlotLayout make_flag_layout(uint32_t Lmax, uint32_t R, uint32_t row_stride, bool hash_smem, uint32_t Scap);
+SlotLayout make_flag_layout(uint32_t Lmax, uint32_t R, uint32_t row_stride, bool hash_smem, uint32_t Scap, bool drop);
 cudaError_t build_flag_search(uint32_t dtype, uint32_t metric, uint32_t grid, uint32_t warps, size_t smem,
                               const BuildFlagArgs &F, int *blocks, cudaStream_t st);
 cudaError_t build_flag_prune(uint32_t dtype, uint32_t metric, uint32_t grid, const BuildFlagArgs &F, const PruneLayout &lay,
@@ -375,7 +375,7 @@ static nbpg_status build_impl(nbpg_index *idx, const nbpg_build_params &P, nbpg_
     F.B.s = sa;
     if (flag) {
         row_geometry(idx->row_stride, 4, F.B.s.vecs, F.B.s.lpr, F.B.s.vpl);
-        flay = make_flag_layout(L, R, idx->row_stride, !ghash, S);
+        flay = make_flag_layout(L, R, idx->row_stride, !ghash, S, false);
         play = make_prune_layout(VL, R, idx->row_stride);
         flag = flay.bytes <= idx->smem_optin && play.bytes <= idx->smem_optin;
     }

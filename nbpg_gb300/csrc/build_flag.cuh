@@ -36,7 +36,7 @@ __device__ __forceinline__ void build_search_one(const BuildFlagArgs &F, uint32_
     const uint32_t index = B.inserts[t];
     const uint8_t *prow = a.base + size_t(index) * a.row_stride;
     // beam search from the start points (beam_search with k = 0, cut = 0)
-    const FlagState st = search_flag<DT, MET, VPL, true, GH>(a, prow, B.L, 0, ~uint64_t(0), B.sp + size_t(t) * B.nsp_per,
+    const FlagState st = search_flag<DT, MET, VPL, true, false, GH>(a, prow, B.L, 0, ~uint64_t(0), B.sp + size_t(t) * B.nsp_per,
                                                              B.nsp_per, slot, gslot, lane, index,
                                                              FlagVisited{F.vis + size_t(t) * FLAG_VIS, B.VL});
     // existing neighbours not seen by the search (nsw.h:150-161); has_been_seen inserts
@@ -47,7 +47,7 @@ __device__ __forceinline__ void build_search_one(const BuildFlagArgs &F, uint32_
     for (uint32_t c = 0; c < deg; c += 32) {
         const bool act = c + lane < deg;
         const uint32_t nb = act ? __ldg(grow + 1 + c + lane) : kNoId;
-        const bool seen = filter_probe(st.H, st.smask, nb, act);  // all lanes
+        const bool seen = filter_probe<GH>(st.H, st.smask, nb, act);  // all lanes
         const bool keep = act && !seen;
         const unsigned km = __ballot_sync(kFull, keep);
         if (keep) filt[nf + __popc(km & lanemask_lt())] = nb;

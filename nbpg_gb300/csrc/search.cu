@@ -64,8 +64,9 @@ SlotLayout make_slot_layout(uint32_t Lmax, uint32_t R, bool vis_smem, uint32_t V
     return l;
 }
 
-// Per-warp slot of search_flag: the query row, one frontier, candidates, the filter, filtered ids.
-SlotLayout make_flag_layout(uint32_t Lmax, uint32_t R, uint32_t row_stride, bool hash_smem, uint32_t Scap)
+// Per-warp slot of search_flag: the query row, one frontier, candidates, the filter, filtered ids; with drop,
+// 32 frontier places past L and the dropped ids.
+SlotLayout make_flag_layout(uint32_t Lmax, uint32_t R, uint32_t row_stride, bool hash_smem, uint32_t Scap, bool drop)
 {
     SlotLayout l{};
     l.Lcap = round_up(std::max<uint32_t>(Lmax, 1), 32);
@@ -74,10 +75,11 @@ SlotLayout make_flag_layout(uint32_t Lmax, uint32_t R, uint32_t row_stride, bool
     l.Scap = hash_smem ? Scap : 0;
     uint32_t off = 0;
     l.off_q = off; off += row_stride;
-    l.off_fr0 = off; off += l.Lcap * 8;
+    l.off_fr0 = off; off += (l.Lcap + (drop ? 32 : 0)) * 8;
     l.off_cand = off; off += l.Ccap * 8;
     l.off_hash = off; off += l.Scap * 4;
     l.off_filt = off; off += l.Rcap * 4;
+    l.off_vis = off; off += drop ? FLAG_DROPS * 4 + FLAG_BLOOM / 8 : 0;
     l.bytes = round_up(off, 16);
     return l;
 }
@@ -147,7 +149,7 @@ static nbpg_status plan_pass_uncached(nbpg_index *idx, const SearchOps *ops, int
     pc.Vcap = round_up(vf * Lmax, 32);
     pc.ghash = !plain && pc.S * 4 > kHashSmemMax;
     pc.gvis = list && !plain && pc.Vcap * 8 > kVisSmemMax;
-    pc.lay = pass == PASS_WIDE ? make_flag_layout(Lmax, R, idx->row_stride, !pc.ghash, pc.S)
+    pc.lay = pass == PASS_WIDE ? make_flag_layout(Lmax, R, idx->row_stride, !pc.ghash, pc.S, metric == M_IP)
                                : make_slot_layout(Lmax, R, list && !pc.gvis, pc.Vcap, !pc.ghash, pc.S);
     if (pc.lay.bytes > idx->smem_optin) {
         set_error("per-query working set exceeds shared memory for this L");
@@ -389,16 +391,16 @@ nbpg_status search_device_impl(nbpg_index *idx, SearchScratch &sc, const void *d
         return NBPG_OK;
     }
     const uint32_t vf = P->visited_factor ? P->visited_factor : 8;
-    // inner product: the cut rule routinely keeps <= k entries, so go straight to LIST;
-    // filtering mode needs the visited list itself
-    const bool flag_first = metric == M_L2 && !(emit && emit->visited);
+    // filtering mode needs the visited list itself; search_flag's inner-product frontier is 32 entries longer
+    // than its 1024 positions allow at the longest beams
+    const bool flag_first = !(emit && emit->visited) && !(metric == M_IP && P->L > 992);
     if (emit && emit->visited)
         NBPG_CHECK_ARG(k_stride >= (P->visited_factor ? P->visited_factor : 8) * P->L,
                        "k_stride must hold the visited list (visited_factor * L)");
 
     PassCfg main{}, rerun{};
-    // beams above 32 (the largest of the call): search_flag's merge, several frontier words
-    const int pass = !flag_first ? PASS_LIST : P->L > 32 ? PASS_WIDE : PASS_FLAG;
+    // beams above 32 (the largest of the call) and inner product: search_flag
+    const int pass = !flag_first ? PASS_LIST : P->L > 32 || metric == M_IP ? PASS_WIDE : PASS_FLAG;
     nbpg_status s = plan_pass(idx, ops, metric, pass, plain, P->L, vf, P->warps_per_cta, main);
     if (s != NBPG_OK) return s;
     if (flag_first) {

@@ -1,7 +1,7 @@
 // Strict greedy beam search with expanded flags instead of a visited list: FLAG mode
 // (search_impl.cuh has the argument why it equals the reference's list), one warp per query.
 //
-// Runs the searches of beams above 32; up to there the frontier is one entry per lane and search_core's
+// Runs the searches of beams above 32 and of inner product; for L2 up to there the frontier is one entry per lane and search_core's
 // merge is as short (10k queries at L = 19 on 1M x 128: 594 us there, 627 here).
 //
 // What bounds it: instructions.  Neither memory nor any pipe is near its limit; a warp spends 5 to 13
@@ -13,9 +13,15 @@
 //     is updated in place, 32 positions at a time from the top down to the first one taken: a position
 //     that no candidate takes gets the entry that the bit counts of the taken ones name, and the same pass
 //     writes the new mask word.  No sort, no search per frontier entry, no second frontier.
+//   - Inner product (DROP): the cut rule keeps next to nothing there, so expanded entries do leave the
+//     frontier and can come back when the filter forgets them.  Their ids are kept, and a candidate found
+//     among them enters as expanded: exactly "frontier minus visited".  More than fit, or a visited cap that
+//     overflows, marks the query for LIST mode.
 //   - The visited filter is probed with an exchange whose read-back shows whether two lanes met in a slot;
 //     only then those lanes are sorted out (a __match_any_sync takes longer than the whole probe).
-// 10k queries at L = 80 on 250k 4-bit rows: 1,196 -> 875 us; 2k re-ranked queries at L = 50: 775 -> 693 us.
+// 10k queries at L = 80 on 250k 4-bit rows: 1,196 -> 875 us; 2k re-ranked queries at L = 50: 775 -> 693 us;
+// 20k inner-product queries of L = 32 .. 256 on 250k x 96 i8 (the visited lists, 16 KB a slot, are gone: 24 warps
+// per SM instead of 10): 2,292 -> 1,056 us.
 #pragma once
 #include "search_impl.cuh"
 
@@ -34,6 +40,9 @@ struct FlagState {
 // Where a build search keeps its expanded keys: room for FLAG_VIS keys in global memory, of which the
 // `keep` smallest stay when it is full.
 constexpr uint32_t FLAG_VIS = 256;
+constexpr uint32_t FLAG_DROPS = 512;   // expanded entries that left the frontier (DROP)
+constexpr uint32_t FLAG_BLOOM = 4096;  // bits that say which ids are surely not among them
+__device__ __forceinline__ uint32_t drop_bit(uint32_t id) { return (id * 0x9E3779B1u) >> 20; }
 struct FlagVisited {
     uint64_t *keys;
     uint32_t keep;
@@ -107,11 +116,23 @@ __device__ __forceinline__ uint32_t flag_row_keys(const SearchArgs &a, const uin
 
 // Probe and insert a chunk of neighbours (lanes with act) in the visited filter, in lane order.
 // Returns whether this lane's id was there.
+// GH: the filter is in global memory, where one round trip costs more than a match.
+template <bool GH>
 __device__ __forceinline__ bool filter_probe(uint32_t *H, uint32_t smask, uint32_t nb, bool act)
 {
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t sl = act ? filter_slot(nb, smask) : kNoId;
     const uint32_t hv = act ? H[sl] : kNoId;
+    if constexpr (GH) {
+        const unsigned here = __match_any_sync(kFull, sl);
+        const unsigned before = here & lanemask_lt();
+        const uint32_t prev = __shfl_sync(kFull, nb, before ? 31 - __clz(before) : int(lane));
+        const bool seen = act && (before ? prev == nb : hv == nb);
+        __syncwarp();
+        if (act && !(here & lanemask_gt())) H[sl] = nb;
+        __syncwarp();
+        return seen;
+    }
     __syncwarp();
     // a slot that one lane holds alone returns what was there; the same id twice in a row returns itself
     // to the later lane: both as the sequential probe sees it
@@ -150,9 +171,32 @@ __device__ __forceinline__ uint32_t count_less(const uint64_t *s, uint32_t n, ui
     return p;
 }
 
-// VIS: keep the expanded keys (v).  GH: the visited filter is a global block, not shared memory (a template
+// Shortens the frontier from fs to `to` entries; the ids of expanded ones among the rest go to drops, as many
+// as fit (nd counts them all).
+__device__ __forceinline__ void flag_drop(const uint64_t *fr, uint32_t &um, uint32_t to, uint32_t &fs, uint32_t *drops,
+                                          uint32_t &nd, int lane)
+{
+    for (uint32_t b = to & ~31u; b < fs; b += 32) {
+        const uint32_t i = b + lane, word = __shfl_sync(kFull, um, int(b >> 5));
+        const bool d = i >= to && i < fs && !((word >> lane) & 1);
+        const unsigned m = __ballot_sync(kFull, d);
+        const uint32_t at = nd + __popc(m & lanemask_lt());
+        if (d) {
+            const uint32_t id = key_id(fr[i]), h = drop_bit(id);
+            if (at < FLAG_DROPS) drops[at] = id;
+            atomicOr(&drops[FLAG_DROPS + (h >> 5)], 1u << (h & 31));
+        }
+        nd += __popc(m);
+    }
+    const uint32_t b = uint32_t(lane) * 32;
+    if (to < b + 32) um &= to > b ? (1u << (to - b)) - 1u : 0u;
+    fs = to;
+    __syncwarp();
+}
+
+// VIS: keep the expanded keys (v).  DROP: expanded entries may leave the frontier (see above).  GH: the visited filter is a global block, not shared memory (a template
 // argument, so that shared-memory probes are not generic accesses).  k = 0: no cut rule.
-template <int DT, int MET, int VPL, bool VIS, bool GH>
+template <int DT, int MET, int VPL, bool VIS, bool DROP, bool GH>
 __device__ FlagState search_flag(const SearchArgs &a, const uint8_t *qrow_bytes, uint32_t L, uint32_t k,
                                  uint64_t max_visited, const uint32_t *sp, uint32_t nsp, uint8_t *slot, uint32_t gslot,
                                  int lane, uint32_t self, FlagVisited v)
@@ -180,19 +224,28 @@ __device__ FlagState search_flag(const SearchArgs &a, const uint8_t *qrow_bytes,
     __syncwarp();
     sort_keys(fr, nsp, lane);
 
+    uint32_t *const drops = reinterpret_cast<uint32_t *>(slot + lay.off_vis);
+    uint32_t nd = 0;
+    bool taint = false;
+    if constexpr (DROP) {
+        for (uint32_t i = lane; i < FLAG_BLOOM / 32; i += 32) drops[FLAG_DROPS + i] = 0;
+        // repeated start points make a multiset of the frontier: LIST mode
+        for (uint32_t i = lane; i + 1 < nsp; i += 32) taint |= fr[i] == fr[i + 1];
+        taint = __any_sync(kFull, taint);
+    }
+
     // lane w: unexpanded entries among positions [32 w, 32 w + 32)
     uint32_t um = nsp >= uint32_t(lane) * 32 + 32 ? kFull : nsp > uint32_t(lane) * 32 ? (1u << (nsp - lane * 32)) - 1u : 0u;
     uint32_t fs = nsp, cmps = nsp, adj = 0, cs = 0, cst = 0, nbuf = 0;
     uint32_t nvis = 0;  // no node is expanded twice, so these fit
     const uint32_t limit = uint32_t(min(a.limit, uint64_t(kNoId))), most = uint32_t(min(max_visited, uint64_t(kNoId)));
-    bool taint = false;
     const uint32_t nchunks = (a.R + 31) / 32;
     const float cut_low = __double2float_rd(a.cut);
     // candidates stored (cst) vs appended (cs, which drives the deferral rule): while the frontier is
     // full, a candidate at or beyond its last key can never survive the union's truncation to L, so it
     // is counted but not stored
     uint64_t tail = fs == L ? fr[L - 1] : kKeyMax;
-    while (nvis < limit) {
+    while (nvis < limit && !(DROP && taint)) {
         const unsigned open = __ballot_sync(kFull, um != 0);
         if (!open) break;
         const int ow = __ffs(open) - 1;
@@ -226,7 +279,7 @@ __device__ FlagState search_flag(const SearchArgs &a, const uint8_t *qrow_bytes,
         for (int c = 0; c < 4; ++c) {
             if (uint32_t(c) * 32 >= ne) break;
             const bool act = uint32_t(c * 32 + lane) < ne;
-            const bool seen = filter_probe(H, smask, nbv[c], act);
+            const bool seen = filter_probe<GH>(H, smask, nbv[c], act);
             const bool keep = act && !seen && nbv[c] != self;
             const unsigned km = __ballot_sync(kFull, keep);
             if (keep) filt[nf + __popc(km & lanemask_lt())] = nbv[c];
@@ -286,7 +339,20 @@ __device__ FlagState search_flag(const SearchArgs &a, const uint8_t *qrow_bytes,
             const bool keep = in && !(p < fs && fr[p] == c) && !(same & lanemask_lt());
             const unsigned km = __ballot_sync(kFull, keep);
             const uint32_t at = keep ? p + __popc(less & km) : kNoId;
-            const uint32_t n0 = min(fs + uint32_t(__popc(km)), L);
+            // (DROP takes the whole union, up to 32 entries past L, and drops the rest below)
+            const uint32_t n0 = DROP ? fs + uint32_t(__popc(km)) : min(fs + uint32_t(__popc(km)), L);
+            unsigned back = 0;  // candidates that were expanded before
+            if constexpr (DROP) {
+                const uint32_t h = drop_bit(key_id(c));
+                bool met = keep && ((drops[FLAG_DROPS + (h >> 5)] >> (h & 31)) & 1);
+                if (__any_sync(kFull, met)) {
+                    const uint32_t kept = min(nd, FLAG_DROPS);
+                    bool there = false;
+                    for (uint32_t j = 0; j < kept; ++j) there |= drops[j] == key_id(c);
+                    met = met && there;
+                }
+                back = __ballot_sync(kFull, met);
+            }
             for (int w = int((n0 - 1) >> 5); w >= 0; --w) {
                 const bool mine = (at >> 5) == uint32_t(w);
                 const uint32_t taken = __reduce_or_sync(kFull, mine ? 1u << (at & 31) : 0u);
@@ -301,11 +367,14 @@ __device__ FlagState search_flag(const SearchArgs &a, const uint8_t *qrow_bytes,
                 __syncwarp();
                 if (old) fr[x] = key;
                 if (mine && at < n0) fr[at] = c;
-                const unsigned bits = __ballot_sync(kFull, x < n0 && (fresh || ((ui >> (i & 31)) & 1)));
+                unsigned bits = __ballot_sync(kFull, x < n0 && (fresh || ((ui >> (i & 31)) & 1)));
+                if (DROP && back) bits &= ~__reduce_or_sync(kFull, mine && ((back >> lane) & 1) ? 1u << (at & 31) : 0u);
                 __syncwarp();
                 if (lane == w) um = bits;
             }
             fs = n0;
+            if constexpr (DROP)
+                if (fs > L) flag_drop(fr, um, L, fs, drops, nd, lane);
         }
         cst = 0;
         // cut rule (beamSearch.h:140-149): threshold = float(cut * d_k), upper_bound of (0, thr)
@@ -331,14 +400,17 @@ __device__ FlagState search_flag(const SearchArgs &a, const uint8_t *qrow_bytes,
                     ub += __popc(__ballot_sync(kFull, pr));
                 }
                 nfs = ub > fs0 ? ub : fs0;
-                if (nfs < fs) {
+                if constexpr (DROP) {
+                    if (nfs < fs) flag_drop(fr, um, nfs, fs, drops, nd, lane);
+                } else if (nfs < fs) {
                     const uint32_t b = uint32_t(lane) * 32;
                     if (nfs < b + 32) um &= nfs > b ? (1u << (nfs - b)) - 1u : 0u;
                     fs = nfs;
                 }
             }
-            if (nfs < k + 1) taint = true;
+            if (!DROP && nfs < k + 1) taint = true;
         }
+        if (DROP && nd > FLAG_DROPS) taint = true;  // some are lost
         tail = fs == L ? fr[L - 1] : kKeyMax;
     }
     FlagState st;

@@ -18,15 +18,15 @@
 //
 // Two modes give the same results as the reference:
 //   LIST  keeps the real capped visited list and computes frontier \ visited by
-//         membership, exactly as the reference.  Used for the build, for
-//         inner product, and as the fallback below.
+//         membership, exactly as the reference.  Used by HNSW, FGIM's pair pass, builds
+//         with VL < L, and as the fallback below.
 //   FLAG  replaces the visited list by an "expanded" bit carried with each frontier
 //         entry.  This equals the reference whenever (a) no expansion overflowed
 //         the visited cap and (b) every merge that applied the cut rule kept more
 //         than k entries (then an entry that left the frontier can never re-enter,
 //         so "in the visited list" == "expanded").  A query that violates (a) or (b)
 //         is marked tainted and re-run in LIST mode by a second launch.
-//         Beams above 32 run FLAG mode in search_flag.cuh.
+//         Beams above 32 and inner product run FLAG mode in search_flag.cuh.
 #pragma once
 #include "common.cuh"
 

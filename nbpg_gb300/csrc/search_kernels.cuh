@@ -1,5 +1,5 @@
-// The strict search kernels: FLAG mode first (search_core, or search_flag for beams above 32), then LIST
-// mode for the queries it marks.
+// The strict search kernels: FLAG mode first (search_core, or search_flag for beams above 32 and for inner
+// product), then LIST mode for the queries it marks.
 #pragma once
 #include "search_flag.cuh"
 
@@ -45,8 +45,8 @@ __device__ void search_query(const SearchArgs &a, uint32_t qi, uint8_t *slot, ui
     uint64_t nvis;
     bool taint;
     if constexpr (PASS == PASS_WIDE) {
-        const FlagState st = search_flag<DT, MET, VPL, false, GH>(a, qrow, L, k, max_visited, sp, nsp, slot, gslot, lane,
-                                                                  kNoId, FlagVisited{});
+        const FlagState st = search_flag<DT, MET, VPL, false, MET == M_IP, GH>(a, qrow, L, k, max_visited, sp, nsp, slot, gslot,
+                                                                               lane, kNoId, FlagVisited{});
         frb = st.fr;
         fs = st.fs, cmps = st.cmps, adj = st.adj, nvis = st.nvis, taint = st.taint;
     } else {

@@ -76,14 +76,18 @@ template <int DT, int VPL>
 struct SearchDispatch {
     static cudaError_t set_attr(int metric, int pass, bool plain, size_t smem)
     {
-        if (metric == M_IP) return set_smem_attr<DT, M_IP, PASS_LIST, VPL>(plain, smem);
+        if (metric == M_IP)
+            return pass == PASS_LIST ? set_smem_attr<DT, M_IP, PASS_LIST, VPL>(plain, smem)
+                                     : set_smem_attr<DT, M_IP, PASS_WIDE, VPL>(plain, smem);
         if (pass == PASS_LIST) return set_smem_attr<DT, M_L2, PASS_LIST, VPL>(plain, smem);
         return pass == PASS_WIDE ? set_smem_attr<DT, M_L2, PASS_WIDE, VPL>(plain, smem)
                                  : set_smem_attr<DT, M_L2, PASS_FLAG, VPL>(plain, smem);
     }
     static cudaError_t occ(int metric, int pass, bool plain, uint32_t threads, size_t smem, int *blocks)
     {
-        if (metric == M_IP) return occupancy<DT, M_IP, PASS_LIST, VPL>(plain, threads, smem, blocks);
+        if (metric == M_IP)
+            return pass == PASS_LIST ? occupancy<DT, M_IP, PASS_LIST, VPL>(plain, threads, smem, blocks)
+                                     : occupancy<DT, M_IP, PASS_WIDE, VPL>(plain, threads, smem, blocks);
         if (pass == PASS_LIST) return occupancy<DT, M_L2, PASS_LIST, VPL>(plain, threads, smem, blocks);
         return pass == PASS_WIDE ? occupancy<DT, M_L2, PASS_WIDE, VPL>(plain, threads, smem, blocks)
                                  : occupancy<DT, M_L2, PASS_FLAG, VPL>(plain, threads, smem, blocks);
@@ -91,7 +95,8 @@ struct SearchDispatch {
     static void launch(int metric, int pass, bool plain, uint32_t grid, uint32_t warps, size_t smem, const SearchArgs &a,
                        cudaStream_t st)
     {
-        if (metric == M_IP) launch_one<DT, M_IP, PASS_LIST, VPL>(plain, grid, warps, smem, a, st);
+        if (metric == M_IP && pass == PASS_LIST) launch_one<DT, M_IP, PASS_LIST, VPL>(plain, grid, warps, smem, a, st);
+        else if (metric == M_IP) launch_one<DT, M_IP, PASS_WIDE, VPL>(plain, grid, warps, smem, a, st);
         else if (pass == PASS_LIST) launch_one<DT, M_L2, PASS_LIST, VPL>(plain, grid, warps, smem, a, st);
         else if (pass == PASS_WIDE) launch_one<DT, M_L2, PASS_WIDE, VPL>(plain, grid, warps, smem, a, st);
         else launch_one<DT, M_L2, PASS_FLAG, VPL>(plain, grid, warps, smem, a, st);

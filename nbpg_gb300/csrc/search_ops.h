@@ -7,7 +7,7 @@
 namespace nbpg {
 
 struct SearchOps {
-    // pass: a SearchPass (FLAG passes are L2 only: inner product goes straight to LIST)
+    // pass: a SearchPass (inner product has no PASS_FLAG)
     cudaError_t (*set_attr)(int metric, int pass, bool plain, size_t smem);
     cudaError_t (*occ)(int metric, int pass, bool plain, uint32_t threads, size_t smem, int *blocks);
     void (*launch)(int metric, int pass, bool plain, uint32_t grid, uint32_t warps, size_t smem, const SearchArgs &a,

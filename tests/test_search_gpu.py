@@ -294,3 +294,32 @@ def test_wide_beams_match_oracle(gpu_lib, oracle_lib, L, R):
         r = idx.search(q, QueryParams(k=k, beamSize=L, cut=cut, limit=limit), start_points=sp, kernel=kernel)
         o = oracle_lib.search("u8", "l2", base, g, q, L=L, k=k, cut=cut, limit=limit or None, start_points=sp)
         _check(r, o, len(q))
+
+
+@pytest.mark.parametrize("R", [8, 33, 64])
+@pytest.mark.parametrize("L", [1, 2, 10, 31, 32, 33, 64, 129, 200, 256, 992, 1000])
+def test_inner_product_drops_match_oracle(gpu_lib, oracle_lib, L, R):
+    """Inner product, where the cut rule drops expanded entries that the lossy filter lets come back: the
+    flags with the dropped ids equal the visited list, queries past their room or with repeated start points
+    take the LIST re-run, beams above 992 LIST alone."""
+    from nbpg_gb300 import synth
+    from nbpg_gb300.index import QueryParams
+    n = 900 if L > 100 else 6000
+    base, q = synth.i8_unit_mixture(n, 24, dim=24, n_centres=12)
+    base[100:140] = base[0:40]
+    g = _rough_graph(n, R, L * 17 + R)
+    idx = _gpu_index(base, g, "i8", "ip")
+    for kernel, cut, k, sp, limit in [("batched", 1.35, 10, (0,), 0), ("plain", 1.0, 1, (5,), 0),
+                                      ("batched", 0.6, 5, (3, 140), 37), ("batched", 0.0, 20, (1,), 0),
+                                      ("batched", 1.35, 3, (7, 7, 8), 0)]:
+        if kernel == "plain" and L > 181:
+            kernel = "batched"
+        if len(sp) > L:
+            continue
+        k = min(k, L)
+        r = idx.search(q, QueryParams(k=k, beamSize=L, cut=cut, limit=limit), start_points=sp, kernel=kernel)
+        o = oracle_lib.search("i8", "ip", base, g, q, L=L, k=k, cut=cut, limit=limit or None, start_points=sp)
+        ids, dists, cnt, vis, cmps = o
+        assert np.array_equal(r.count, cnt) and np.array_equal(r.ids, ids), (kernel, cut)
+        assert np.array_equal(r.dists.view(np.uint32), dists.view(np.uint32))
+        assert np.array_equal(r.visited, vis) and np.array_equal(r.cmps, cmps)
