@@ -114,52 +114,6 @@ __device__ __forceinline__ uint32_t flag_row_keys(const SearchArgs &a, const uin
     return FILTER ? stored : cnt;
 }
 
-// Probe and insert a chunk of neighbours (lanes with act) in the visited filter, in lane order.
-// Returns whether this lane's id was there.
-// GH: the filter is in global memory, where one round trip costs more than a match.
-template <bool GH>
-__device__ __forceinline__ bool filter_probe(uint32_t *H, uint32_t smask, uint32_t nb, bool act)
-{
-    const uint32_t lane = threadIdx.x & 31;
-    const uint32_t sl = act ? filter_slot(nb, smask) : kNoId;
-    const uint32_t hv = act ? H[sl] : kNoId;
-    if constexpr (GH) {
-        const unsigned here = __match_any_sync(kFull, sl);
-        const unsigned before = here & lanemask_lt();
-        const uint32_t prev = __shfl_sync(kFull, nb, before ? 31 - __clz(before) : int(lane));
-        const bool seen = act && (before ? prev == nb : hv == nb);
-        __syncwarp();
-        if (act && !(here & lanemask_gt())) H[sl] = nb;
-        __syncwarp();
-        return seen;
-    }
-    __syncwarp();
-    // a slot that one lane holds alone returns what was there; the same id twice in a row returns itself
-    // to the later lane: both as the sequential probe sees it
-    const uint32_t old = act ? atomicExch(&H[sl], nb) : kNoId;
-    __syncwarp();
-    bool seen = act && old == nb;
-    // different ids in one slot (32 ids: one time in three at 1,024 slots, one in nine at 4,096): the last
-    // earlier lane there decides, the last lane stays
-    unsigned lost = __ballot_sync(kFull, act && H[sl] != nb);
-    if (lost) {
-        __syncwarp();
-        while (lost) {
-            const uint32_t s = __shfl_sync(kFull, sl, __ffs(lost) - 1);
-            const unsigned here = __ballot_sync(kFull, sl == s);
-            const unsigned before = here & lanemask_lt();
-            const uint32_t prev = __shfl_sync(kFull, nb, before ? 31 - __clz(before) : int(lane));
-            if (sl == s) {
-                seen = before ? prev == nb : hv == nb;
-                if (!(here & lanemask_gt())) H[sl] = nb;
-            }
-            lost &= ~here;
-        }
-    }
-    __syncwarp();
-    return seen;
-}
-
 // Entries of sorted s[0, n) that are < key, without branches (n <= 1024)
 __device__ __forceinline__ uint32_t count_less(const uint64_t *s, uint32_t n, uint64_t key)
 {

@@ -294,6 +294,52 @@ __device__ __forceinline__ uint32_t warp_upper_bound(const uint64_t *s, uint32_t
     return n;
 }
 
+// Probe and insert a chunk of neighbours (lanes with act) in the visited filter, in lane order.
+// Returns whether this lane's id was there.
+// GH: the filter may be in global memory, where one round trip costs more than a match.
+template <bool GH>
+__device__ __forceinline__ bool filter_probe(uint32_t *H, uint32_t smask, uint32_t nb, bool act)
+{
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t sl = act ? filter_slot(nb, smask) : kNoId;
+    const uint32_t hv = act ? H[sl] : kNoId;
+    if constexpr (GH) {
+        const unsigned here = __match_any_sync(kFull, sl);
+        const unsigned before = here & lanemask_lt();
+        const uint32_t prev = __shfl_sync(kFull, nb, before ? 31 - __clz(before) : int(lane));
+        const bool seen = act && (before ? prev == nb : hv == nb);
+        __syncwarp();
+        if (act && !(here & lanemask_gt())) H[sl] = nb;
+        __syncwarp();
+        return seen;
+    }
+    __syncwarp();
+    // a slot that one lane holds alone returns what was there; the same id twice in a row returns itself
+    // to the later lane: both as the sequential probe sees it
+    const uint32_t old = act ? atomicExch(&H[sl], nb) : kNoId;
+    __syncwarp();
+    bool seen = act && old == nb;
+    // different ids in one slot (32 ids: one time in three at 1,024 slots, one in nine at 4,096): the last
+    // earlier lane there decides, the last lane stays
+    unsigned lost = __ballot_sync(kFull, act && H[sl] != nb);
+    if (lost) {
+        __syncwarp();
+        while (lost) {
+            const uint32_t s = __shfl_sync(kFull, sl, __ffs(lost) - 1);
+            const unsigned here = __ballot_sync(kFull, sl == s);
+            const unsigned before = here & lanemask_lt();
+            const uint32_t prev = __shfl_sync(kFull, nb, before ? 31 - __clz(before) : int(lane));
+            if (sl == s) {
+                seen = before ? prev == nb : hv == nb;
+                if (!(here & lanemask_gt())) H[sl] = nb;
+            }
+            lost &= ~here;
+        }
+    }
+    __syncwarp();
+    return seen;
+}
+
 // The search itself (filtered_beam_search with Points == Q_Points), executed by the
 // whole warp on one query row.  slot: this warp's shared-memory slot; gslot: index of
 // its global scratch block; sp/nsp: start points; self: node excluded from expansion
@@ -334,7 +380,9 @@ __device__ SearchState search_core(const SearchArgs &a, const uint8_t *qrow_byte
     if constexpr (LIST)
         vis = a.g_vis ? a.g_vis + size_t(gslot) * a.g_vis_cap : reinterpret_cast<uint64_t *>(slot + lay.off_vis);
     st.vis = vis;
-    uint32_t *H = a.g_hash ? a.g_hash + size_t(gslot) * a.g_hash_slots : reinterpret_cast<uint32_t *>(slot + lay.off_hash);
+    // (FLAG mode here runs beams whose filter fits in shared memory: no generic accesses then)
+    uint32_t *H = LIST && a.g_hash ? a.g_hash + size_t(gslot) * a.g_hash_slots
+                                   : reinterpret_cast<uint32_t *>(slot + lay.off_hash);
     st.H = H;
 
     // query vector in registers: this lane's 16-byte pieces of the row
@@ -391,6 +439,7 @@ __device__ SearchState search_core(const SearchArgs &a, const uint8_t *qrow_byte
     bool taint = false;
     const uint32_t R = a.R;
     const uint32_t nchunks = (R + 31) / 32;
+    const float cut_low = __double2float_rd(a.cut);
 
     // candidates stored (cst) vs appended (cs, which drives the deferral rule): while the
     // frontier is full, a candidate at or beyond its last key can never survive the
@@ -432,16 +481,7 @@ __device__ SearchState search_core(const SearchArgs &a, const uint8_t *qrow_byte
             const uint32_t i = c * 32 + lane;
             const bool act = i < ne;
             const uint32_t nb = nbv[c];
-            const uint32_t sl = act ? filter_slot(nb, smask) : 0xFFFFFFFFu;
-            const unsigned peers = __match_any_sync(kFull, sl);
-            const unsigned earlier = peers & lanemask_lt();
-            const int src = earlier ? 31 - __clz(earlier) : lane;
-            const uint32_t prev_nb = __shfl_sync(kFull, nb, src);
-            const uint32_t hv = (act && !earlier) ? H[sl] : kNoId;
-            const bool seen = act && (earlier ? (prev_nb == nb) : (hv == nb));
-            __syncwarp();
-            if (act && !(peers & lanemask_gt())) H[sl] = nb;
-            __syncwarp();
+            const bool seen = LIST ? filter_probe<true>(H, smask, nb, act) : filter_probe<false>(H, smask, nb, act);
             const bool keep = act && !seen && nb != self;
             const unsigned km = __ballot_sync(kFull, keep);
             if (keep) filt[nf + __popc(km & lanemask_lt())] = nb;
@@ -530,22 +570,29 @@ __device__ SearchState search_core(const SearchArgs &a, const uint8_t *qrow_byte
         uint32_t nfs = n0;
         // cut rule (beamSearch.h:140-149): threshold = float(cut * d_k), upper_bound of (0, thr)
         if (k > 0 && n0 > k) {
-            // the one double product of the loop, on one lane (FP64 issue is scarce on this part)
-            float thr = 0.f;
-            if (lane == 0) thr = __double2float_rn(a.cut * double(key_dist(frn[k])));
-            thr = __shfl_sync(kFull, thr, 0);
-            uint32_t ub = 0;
-            for (uint32_t base = 0; base < n0; base += 32) {
-                const uint32_t i = base + lane;
-                bool pr = false;
-                if (i < n0) {
-                    const uint64_t key = frn[i];
-                    const float d = key_dist(key);
-                    pr = d < thr || (d == thr && key_id(key) == 0);
+            const float dk = key_dist(frn[k]), dlast = key_dist(frn[n0 - 1]);
+            // nothing to cut when the last distance lies below a product rounded down at both steps (squared
+            // distances are not negative): the double product is needed only near the threshold
+            if (MET == M_L2 && dlast < __fmul_rd(cut_low, dk)) {
+                nfs = n0;
+            } else {
+                // on one lane: FP64 issue is scarce on this part
+                float thr = 0.f;
+                if (lane == 0) thr = __double2float_rn(a.cut * double(dk));
+                thr = __shfl_sync(kFull, thr, 0);
+                uint32_t ub = 0;
+                for (uint32_t base = 0; base < n0; base += 32) {
+                    const uint32_t i = base + lane;
+                    bool pr = false;
+                    if (i < n0) {
+                        const uint64_t key = frn[i];
+                        const float d = key_dist(key);
+                        pr = d < thr || (d == thr && key_id(key) == 0);
+                    }
+                    ub += __popc(__ballot_sync(kFull, pr));
                 }
-                ub += __popc(__ballot_sync(kFull, pr));
+                nfs = ub > fs ? ub : fs;
             }
-            nfs = ub > fs ? ub : fs;
             if (nfs < k + 1) taint = true;
         }
         b = nb2;
