@@ -371,6 +371,7 @@ static nbpg_status build_impl(nbpg_index *idx, const nbpg_build_params &P, nbpg_
     SlotLayout flay{};
     PruneLayout play{};
     uint32_t fw = 0, fgrid = 0;  // warps per CTA, CTAs
+    size_t fsmem = 0;
     BuildFlagArgs F{};
     F.B.s = sa;
     if (flag) {
@@ -380,15 +381,22 @@ static nbpg_status build_impl(nbpg_index *idx, const nbpg_build_params &P, nbpg_
         flag = flay.bytes <= idx->smem_optin && play.bytes <= idx->smem_optin;
     }
     if (flag) {
+        // 16 warps per CTA: those whose filter fits in shared memory, the rest with theirs in global memory
+        // (slower by the probes' round trips, but a batch's last inserts no longer wait for a second turn)
+        F.lay_g = make_flag_layout(L, R, idx->row_stride, false, S, false);
+        F.own = ghash ? 0 : std::min<uint32_t>(16, uint32_t(idx->smem_optin / flay.bytes));
+        const size_t left = idx->smem_optin - F.own * size_t(flay.bytes);
+        const uint32_t out = std::min<uint32_t>(16 - F.own, uint32_t(left / F.lay_g.bytes));
+        fw = F.own + out;
+        fsmem = F.own * size_t(flay.bytes) + out * size_t(F.lay_g.bytes);
         int fb = 0;
-        fw = std::min<uint32_t>(16, uint32_t(idx->smem_optin / flay.bytes));
-        NBPG_CUDA_TRY(build_flag_search(idx->desc.dtype, idx->desc.metric, 0, fw, fw * size_t(flay.bytes), F, &fb, st));
+        NBPG_CUDA_TRY(build_flag_search(idx->desc.dtype, idx->desc.metric, 0, fw, fsmem, F, &fb, st));
         NBPG_CUDA_TRY(build_flag_prune(idx->desc.dtype, idx->desc.metric, 0, F, play, st));
         flag = fb >= 1;
         fgrid = uint32_t(fb) * uint32_t(idx->sm_count);
-        if (flag && ghash) {
-            if ((s = idx->ghash.ensure(std::max(nslots, size_t(fgrid) * fw) * S * 4)) != NBPG_OK) return s;
-            sa.g_hash = idx->ghash.as<uint32_t>();
+        if (flag && out) {
+            if ((s = idx->ghash.ensure(std::max(ghash ? nslots : 0, size_t(fgrid) * out) * S * 4)) != NBPG_OK) return s;
+            if (ghash) sa.g_hash = idx->ghash.as<uint32_t>();
         }
     }
 
@@ -547,8 +555,10 @@ static nbpg_status build_impl(nbpg_index *idx, const nbpg_build_params &P, nbpg_
                 F.B.s.lpr = geometry.lpr;
                 F.B.s.vpl = geometry.vpl;
                 F.B.s.lay = flay;
+                F.B.s.g_hash = idx->ghash.as<uint32_t>();
+                F.B.s.g_hash_slots = S;
                 const uint32_t gf = std::min<uint32_t>(fgrid, (bs + fw - 1) / fw);
-                NBPG_CUDA_TRY(build_flag_search(idx->desc.dtype, idx->desc.metric, gf, fw, fw * size_t(flay.bytes), F, nullptr, st));
+                NBPG_CUDA_TRY(build_flag_search(idx->desc.dtype, idx->desc.metric, gf, fw, fsmem, F, nullptr, st));
                 NBPG_CUDA_TRY(build_flag_prune(idx->desc.dtype, idx->desc.metric, bs, F, play, st));
             } else {
                 kt.search(g1, W * 32, smem_search, B, st);

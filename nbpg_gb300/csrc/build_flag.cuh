@@ -9,11 +9,11 @@
 // the VL smallest expanded keys, sorted once, by the second kernel.
 //
 // Why two kernels: the search is bound by the latency of its chain of expansions, in a slot whose visited
-// filter (16 KB at L = 100) limits it to 12 warps per SM; the prune is bound by its rounds, each a pivot
+// filter (16 KB at L = 100) limits it to 12 warps per SM, so four more keep theirs in global memory; the prune is bound by its rounds, each a pivot
 // against all candidates left, which four warps share, with the candidates' rows staged in shared memory.
 // RobustPrune takes one barrier per round: the survivors are a bitmask.
 // A 2,000-insert batch of a 100k x 128 build (L = 100, VL = 140): 1.55 ms in one kernel, one warp per insert and
-// LIST search; 0.47 + 0.14 ms here.
+// LIST search; 0.38 + 0.14 ms here (the search took 0.47 with the 12 warps of the shared-memory filters alone).
 #pragma once
 #include "build_impl.cuh"
 #include "search_flag.cuh"
@@ -25,11 +25,14 @@ struct BuildFlagArgs {
     uint64_t *vis;   // [insert][FLAG_VIS] expanded keys, unsorted
     uint64_t *near;  // [insert][R] keys of the node's neighbours that the search did not see
     uint4 *info;     // [insert] expanded keys kept, neighbours, distances, expansions
+    uint32_t own;    // warps of a CTA with the visited filter in shared memory; the others' is in global memory
+    SlotLayout lay_g;  // and their slot
 };
 
 // Persistent warps over the batch's inserts.
 template <int DT, int MET, int VPL, bool GH>
-__device__ __forceinline__ void build_search_one(const BuildFlagArgs &F, uint32_t t, uint8_t *slot, uint32_t gslot, int lane)
+__device__ __forceinline__ void build_search_one(const BuildFlagArgs &F, uint32_t t, const SlotLayout &lay, uint8_t *slot,
+                                                 uint32_t gslot, int lane)
 {
     const BuildArgs &B = F.B;
     const SearchArgs &a = B.s;
@@ -37,10 +40,10 @@ __device__ __forceinline__ void build_search_one(const BuildFlagArgs &F, uint32_
     const uint8_t *prow = a.base + size_t(index) * a.row_stride;
     // beam search from the start points (beam_search with k = 0, cut = 0)
     const FlagState st = search_flag<DT, MET, VPL, true, false, GH>(a, prow, B.L, 0, ~uint64_t(0), B.sp + size_t(t) * B.nsp_per,
-                                                             B.nsp_per, slot, gslot, lane, index,
+                                                             B.nsp_per, lay, slot, gslot, lane, index,
                                                              FlagVisited{F.vis + size_t(t) * FLAG_VIS, B.VL});
     // existing neighbours not seen by the search (nsw.h:150-161); has_been_seen inserts
-    uint32_t *filt = reinterpret_cast<uint32_t *>(slot + a.lay.off_filt);
+    uint32_t *filt = reinterpret_cast<uint32_t *>(slot + lay.off_filt);
     const uint32_t *grow = a.graph + size_t(index) * a.gstride;
     const uint32_t deg = __ldg(grow);
     uint32_t nf = 0;
@@ -54,7 +57,7 @@ __device__ __forceinline__ void build_search_one(const BuildFlagArgs &F, uint32_
         nf += __popc(km);
     }
     __syncwarp();
-    flag_row_keys<DT, MET, VPL, false>(a, reinterpret_cast<const uint4 *>(slot + a.lay.off_q), filt, nf,
+    flag_row_keys<DT, MET, VPL, false>(a, reinterpret_cast<const uint4 *>(slot + lay.off_q), filt, nf,
                                        F.near + size_t(t) * B.R, 0, lane);
     if (lane == 0) F.info[t] = make_uint4(st.nbuf, nf, st.cmps + nf, st.nvis);
     __syncwarp();
@@ -65,15 +68,17 @@ __global__ void __launch_bounds__(512) build_search_kernel(BuildFlagArgs F)
 {
     extern __shared__ __align__(16) uint8_t smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    uint8_t *slot = smem + size_t(warp) * F.B.s.lay.bytes;
-    const uint32_t gslot = blockIdx.x * (blockDim.x >> 5) + warp;
+    const bool own = uint32_t(warp) < F.own;
+    const uint32_t out = uint32_t(warp) - F.own;  // index among the others
+    uint8_t *slot = smem + (own ? size_t(warp) * F.B.s.lay.bytes : size_t(F.own) * F.B.s.lay.bytes + size_t(out) * F.lay_g.bytes);
+    const uint32_t gslot = blockIdx.x * ((blockDim.x >> 5) - F.own) + out;
     while (true) {
         uint32_t w = 0;
         if (lane == 0) w = atomicAdd(F.B.queue, 1u);
         w = __shfl_sync(kFull, w, 0);
         if (w >= F.B.bs) break;
-        if (F.B.s.g_hash) build_search_one<DT, MET, VPL, true>(F, w, slot, gslot, lane);
-        else build_search_one<DT, MET, VPL, false>(F, w, slot, gslot, lane);
+        if (own) build_search_one<DT, MET, VPL, false>(F, w, F.B.s.lay, slot, 0, lane);
+        else build_search_one<DT, MET, VPL, true>(F, w, F.lay_g, slot, gslot, lane);
     }
 }
 

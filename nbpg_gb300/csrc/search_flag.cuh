@@ -152,10 +152,9 @@ __device__ __forceinline__ void flag_drop(const uint64_t *fr, uint32_t &um, uint
 // argument, so that shared-memory probes are not generic accesses).  k = 0: no cut rule.
 template <int DT, int MET, int VPL, bool VIS, bool DROP, bool GH>
 __device__ FlagState search_flag(const SearchArgs &a, const uint8_t *qrow_bytes, uint32_t L, uint32_t k,
-                                 uint64_t max_visited, const uint32_t *sp, uint32_t nsp, uint8_t *slot, uint32_t gslot,
-                                 int lane, uint32_t self, FlagVisited v)
+                                 uint64_t max_visited, const uint32_t *sp, uint32_t nsp, const SlotLayout &lay,
+                                 uint8_t *slot, uint32_t gslot, int lane, uint32_t self, FlagVisited v)
 {
-    const SlotLayout &lay = a.lay;
     const uint32_t S = filter_slots_for(L), smask = S - 1;
     uint64_t *const fr = reinterpret_cast<uint64_t *>(slot + lay.off_fr0);
     uint64_t *const cand = reinterpret_cast<uint64_t *>(slot + lay.off_cand);

@@ -45,8 +45,8 @@ __device__ void search_query(const SearchArgs &a, uint32_t qi, uint8_t *slot, ui
     uint64_t nvis;
     bool taint;
     if constexpr (PASS == PASS_WIDE) {
-        const FlagState st = search_flag<DT, MET, VPL, false, MET == M_IP, GH>(a, qrow, L, k, max_visited, sp, nsp, slot, gslot,
-                                                                               lane, kNoId, FlagVisited{});
+        const FlagState st = search_flag<DT, MET, VPL, false, MET == M_IP, GH>(a, qrow, L, k, max_visited, sp, nsp, a.lay, slot,
+                                                                               gslot, lane, kNoId, FlagVisited{});
         frb = st.fr;
         fs = st.fs, cmps = st.cmps, adj = st.adj, nvis = st.nvis, taint = st.taint;
     } else {
