@@ -78,12 +78,12 @@ struct ReleaseOnExit {
 // list, start points, and global visited-filter / visited-list blocks for large L.
 // Launches that may overlap on the device need separate scratch.
 struct SearchScratch {
-    DevBuf queue, taint, sp, ghash, gvis;
+    DevBuf queue, sp, ghash, gvis;
     const uint32_t *order = nullptr;  // optional processing order of the next launch (device)
     std::vector<uint32_t> sp_host;  // start points currently in `sp`
     void release()
     {
-        for (DevBuf *b : {&queue, &taint, &sp, &ghash, &gvis}) b->release();
+        for (DevBuf *b : {&queue, &sp, &ghash, &gvis}) b->release();
         sp_host.clear();
     }
 };
