@@ -93,7 +93,7 @@ cudaError_t build_flag_prune(uint32_t dtype, uint32_t metric, uint32_t grid, con
 // and adds them to its neighbours' totals, so a node keeps what later nodes add: its visits plus those of the
 // in-neighbours with larger ids.  Visits are counts, and float sums of them are exact in any order below
 // 2^24: there the device adds them, as integers.  (A total at or past 2^24 or a self-loop, and the
-// host walks as the reference does.)  The host's copy of the graph and its walk took 14 of the 227 ms of a
+// host walks as the reference does; so it does where the sums do not fit.)  The host's copy of the graph and its walk took 14 of the 227 ms of a
 // 250k-row build.
 // ---------------------------------------------------------------------------
 static __global__ void __launch_bounds__(256) popular_spread_kernel(const uint32_t *graph, uint32_t gstride, uint32_t n,
@@ -431,7 +431,11 @@ static nbpg_status build_impl(nbpg_index *idx, const nbpg_build_params &P, nbpg_
         flag = fb >= 1;
         fgrid = uint32_t(fb) * uint32_t(idx->sm_count);
         if (flag && out) {
-            if ((s = idx->ghash.ensure(std::max(ghash ? nslots : 0, size_t(fgrid) * out) * S * 4)) != NBPG_OK) return s;
+            if (idx->ghash.ensure(std::max(ghash ? nslots : 0, size_t(fgrid) * out) * S * 4) != NBPG_OK) {
+                cudaGetLastError();  // no room: the one-kernel insert needs less
+                flag = false;
+                if (ghash && (s = idx->ghash.ensure(nslots * S * 4)) != NBPG_OK) return s;
+            }
             if (ghash) sa.g_hash = idx->ghash.as<uint32_t>();
         }
     }
@@ -467,8 +471,9 @@ static nbpg_status build_impl(nbpg_index *idx, const nbpg_build_params &P, nbpg_
     }
 
     if (flag) {
-        if ((s = d_vis.ensure(eff * FLAG_VIS * 8)) || (s = d_near.ensure(eff * R * 8)) || (s = d_info.ensure(eff * 16)))
-            return fail_oom(s);
+        flag = d_vis.ensure(eff * FLAG_VIS * 8) == NBPG_OK && d_near.ensure(eff * R * 8) == NBPG_OK &&
+               d_info.ensure(eff * 16) == NBPG_OK;
+        if (!flag) cudaGetLastError();
         F.vis = d_vis.as<uint64_t>();
         F.near = d_near.as<uint64_t>();
         F.info = d_info.as<uint4>();
@@ -634,18 +639,23 @@ static nbpg_status build_impl(nbpg_index *idx, const nbpg_build_params &P, nbpg_
             std::vector<float> tmp(n, 0.0f);
             DevBuf d_sum, d_total;
             ReleaseOnExit release_pop{{&d_sum, &d_total}};
-            if ((s = d_sum.ensure(n * 8 + 4)) || (s = d_total.ensure(n * 4))) return s;
-            auto *sum = d_sum.as<unsigned long long>();
-            uint32_t *d_inexact = reinterpret_cast<uint32_t *>(sum + n), inexact = 0;
-            NBPG_CUDA_TRY(cudaMemsetAsync(sum, 0, n * 8 + 4, st));
-            popular_spread_kernel<<<uint32_t(idx->sm_count) * 8, 256, 0, st>>>(wg, idx->gstride, uint32_t(n), d_pop.as<float>(),
-                                                                              sum, d_inexact);
-            popular_total_kernel<<<uint32_t((n + 255) / 256), 256, 0, st>>>(uint32_t(n), d_pop.as<float>(), sum,
-                                                                           d_total.as<float>(), d_inexact);
-            NBPG_CUDA_TRY(cudaGetLastError());
-            NBPG_CUDA_TRY(cudaMemcpyAsync(tmp.data(), d_total.ptr, n * 4, cudaMemcpyDeviceToHost, st));
-            NBPG_CUDA_TRY(cudaMemcpyAsync(&inexact, d_inexact, 4, cudaMemcpyDeviceToHost, st));
-            NBPG_CUDA_TRY(cudaStreamSynchronize(st));
+            uint32_t inexact = 0;
+            if (d_sum.ensure(n * 8 + 4) != NBPG_OK || d_total.ensure(n * 4) != NBPG_OK) {
+                cudaGetLastError();
+                inexact = 1;
+            } else {
+                auto *sum = d_sum.as<unsigned long long>();
+                uint32_t *d_inexact = reinterpret_cast<uint32_t *>(sum + n);
+                NBPG_CUDA_TRY(cudaMemsetAsync(sum, 0, n * 8 + 4, st));
+                popular_spread_kernel<<<uint32_t(idx->sm_count) * 8, 256, 0, st>>>(wg, idx->gstride, uint32_t(n),
+                                                                                  d_pop.as<float>(), sum, d_inexact);
+                popular_total_kernel<<<uint32_t((n + 255) / 256), 256, 0, st>>>(uint32_t(n), d_pop.as<float>(), sum,
+                                                                               d_total.as<float>(), d_inexact);
+                NBPG_CUDA_TRY(cudaGetLastError());
+                NBPG_CUDA_TRY(cudaMemcpyAsync(tmp.data(), d_total.ptr, n * 4, cudaMemcpyDeviceToHost, st));
+                NBPG_CUDA_TRY(cudaMemcpyAsync(&inexact, d_inexact, 4, cudaMemcpyDeviceToHost, st));
+                NBPG_CUDA_TRY(cudaStreamSynchronize(st));
+            }
             if (inexact) {
                 std::vector<float> pop(n);
                 std::vector<uint32_t> G(size_t(n) * (R + 1));
