@@ -9,9 +9,10 @@
 // the VL smallest expanded keys, sorted once, by the second kernel.
 //
 // Why two kernels: the search is bound by the latency of its chain of expansions, in a slot whose visited
-// filter (16 KB at L = 100) limits it to 12 warps per SM, so four more keep theirs in global memory; the prune is bound by its rounds, each a pivot
-// against all candidates left, which four warps share, with the candidates' rows staged in shared memory.
-// RobustPrune takes one barrier per round: the survivors are a bitmask.
+// filter (16 KB at L = 100) limits it to 12 warps per SM, so four more keep theirs in global memory; the prune
+// is bound by its rounds, each a pivot against all candidates left, which four warps share, with the
+// candidates' rows staged in shared memory.  RobustPrune takes one barrier per round: the survivors are a
+// bitmask.
 // A 2,000-insert batch of a 100k x 128 build (L = 100, VL = 140): 1.55 ms in one kernel, one warp per insert and
 // LIST search; 0.38 + 0.14 ms here (the search took 0.47 with the 12 warps of the shared-memory filters alone).
 #pragma once

@@ -7,6 +7,7 @@
 //      neighbours not yet seen, merge_union with the visited list, sort_candidates,
 //      RobustPrune (nsw.h:122-175, prune.h:50-87,159-209).  Visited entries are
 //      counted into `popular` in a popularity pass (nsw.h:220-230).
+//      The flat build with VL >= L runs two kernels instead (build_flag.cuh).
 //   2. forward_write_kernel       G[index] = pruned list (nsw.h:416-429).
 //   3-5. reverse edges grouped by target without a sort: atomic per-target counts
 //      give each edge its rank, the first edge of each target bump-allocates a

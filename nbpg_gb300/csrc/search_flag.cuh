@@ -1,8 +1,9 @@
 // Strict greedy beam search with expanded flags instead of a visited list: FLAG mode
 // (search_impl.cuh has the argument why it equals the reference's list), one warp per query.
 //
-// Runs the searches of beams above 32 and of inner product; for L2 up to there the frontier is one entry per lane and search_core's
-// merge is as short (10k queries at L = 19 on 1M x 128: 594 us there, 627 here).
+// Runs the searches of beams above 32 and of inner product.  For L2 up to there the frontier is one entry per
+// lane and search_core's merge is as short (10k queries at L = 19 on 1M x 128: 594 us there, 627 here; 556
+// there since its filter probe is an exchange as well and its cut threshold is computed only where it matters).
 //
 // What bounds it: instructions.  Neither memory nor any pipe is near its limit; a warp spends 5 to 13
 // cycles on each dependent instruction, so what counts is how many an expansion takes.
