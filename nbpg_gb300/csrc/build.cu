@@ -734,13 +734,14 @@ static nbpg_status build_impl(nbpg_index *idx, const nbpg_build_params &P, nbpg_
         d_tog.release();
     }
 
-    uint64_t iso = 0;
-    if (P.repair_isolate) {
-        if ((s = repair_isolated(idx, 0, &iso)) != NBPG_OK) return s;
-    }
     if (out_sv) NBPG_CUDA_TRY(cudaMemcpyAsync(out_sv, d_sv.ptr, n * 4, cudaMemcpyDeviceToHost, st));
     if (out_sd) NBPG_CUDA_TRY(cudaMemcpyAsync(out_sd, d_sd.ptr, n * 4, cudaMemcpyDeviceToHost, st));
     NBPG_CUDA_TRY(cudaStreamSynchronize(st));
+    uint64_t iso = 0;
+    if (P.repair_isolate) {
+        for (DevBuf *b : release_bufs.bufs) b->release();  // the repair's rows find room where the batches' were
+        if ((s = repair_isolated(idx, 0, &iso)) != NBPG_OK) return s;
+    }
     if (stats) {
         stats->isolated = iso;
         stats->batches = batches;
