@@ -226,10 +226,12 @@ extern "C" nbpg_status nbpg_search_rerank(nbpg_index *idx, const void *queries, 
     ReleaseOnExit release_work{{&work}};
     const size_t qbytes = size_t(nq) * idx->row_stride, rqbytes = size_t(nq) * rb;
     const size_t cand_b = size_t(nq) * cs * 4, outb = size_t(nq) * k_stride * 4;
-    nbpg_status s = work.ensure(qbytes + rqbytes + 2 * cand_b + outb * 2 + size_t(nq) * 4 * 6 + 1024);
+    // 11 pieces in steps of 256 bytes
+    auto step = [](size_t b) { return (b + 255) / 256 * 256; };
+    nbpg_status s = work.ensure(step(qbytes) + step(rqbytes) + 2 * step(cand_b) + 2 * step(outb) + 5 * step(size_t(nq) * 4));
     if (s != NBPG_OK) return s;
     uint8_t *w = static_cast<uint8_t *>(work.ptr);
-    auto take = [&](size_t b) { uint8_t *p = w; w += (b + 255) / 256 * 256; return p; };
+    auto take = [&](size_t b) { uint8_t *p = w; w += step(b); return p; };
     uint8_t *dq = take(qbytes), *drq = take(rqbytes);
     uint32_t *d_cand = reinterpret_cast<uint32_t *>(take(cand_b));
     float *d_cd = reinterpret_cast<float *>(take(cand_b));

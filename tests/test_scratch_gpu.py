@@ -1,0 +1,52 @@
+"""Device memory and shared-memory limits as the library asks the CUDA runtime for them: child processes with
+tests/runtime_shim.c between the two."""
+import os
+import subprocess
+import sys
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+HEAD = """
+import ctypes as C, sys
+import numpy as np
+sys.path[:0] = [{root!r}, {here!r}]
+shim = C.CDLL(None)
+shim.shim_limit.argtypes = [C.c_size_t]
+shim.shim_used.restype = shim.shim_peak.restype = C.c_size_t
+from nbpg_gb300 import _lib, synth
+from nbpg_gb300.index import Index, LaunchConfig, QueryParams, ground_truth
+r = np.random.default_rng(3)
+""".format(root=os.path.dirname(HERE), here=HERE)
+
+
+@pytest.fixture(scope="session")
+def shim(gpu_lib, tmp_path_factory):
+    so = tmp_path_factory.mktemp("shim") / "shim.so"
+    subprocess.run(["gcc", "-O1", "-shared", "-fPIC", "-o", str(so), os.path.join(HERE, "runtime_shim.c"), "-ldl",
+                    "-lpthread"], check=True)
+
+    def run(code):
+        p = subprocess.run([sys.executable, "-c", HEAD + code], env=dict(os.environ, LD_PRELOAD=str(so)),
+                           capture_output=True, text=True, timeout=300)
+        assert p.returncode == 0, p.stdout[-2000:] + p.stderr[-3000:]
+    return run
+
+
+def test_rerank_of_one_short_query_stays_in_its_scratch(shim):
+    shim("""
+base = r.integers(0, 256, (500, 16)).astype(np.uint8)
+raw = r.normal(size=(500, 5)).astype(np.float32)
+idx = Index(base, "u8", "l2", max_degree=16)
+idx.build_vamana(L=24, VL=32, num_split=0, num_passes=1)
+idx.set_raw_points(raw)
+qp = QueryParams(k=1, beamSize=16)
+many = idx.search_rerank(base[:64], raw[:64], qp, 1)
+for i in range(3):
+    one = idx.search_rerank(base[i:i + 1], raw[i:i + 1], qp, 1)
+    assert one.ids[0, 0] == many.ids[i, 0] and one.dists[0, 0] == many.dists[i, 0]
+idx.close()
+assert shim.shim_peak() > 0 and shim.shim_overrun() == 0
+""")
