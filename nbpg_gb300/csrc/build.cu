@@ -28,12 +28,8 @@ template <int DT, int MET, int VPL>
 struct BuildKernels {
     static cudaError_t setup(size_t smem_search, size_t smem_merge)
     {
-        cudaError_t e = cudaFuncSetAttribute(build_search_prune_kernel<DT, MET, VPL>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem_search));
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(rev_merge_kernel<DT, MET, VPL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     int(smem_merge));
-        return e;
+        const cudaError_t e = raise_smem_limit(build_search_prune_kernel<DT, MET, VPL>, smem_search);
+        return e == cudaSuccess ? raise_smem_limit(rev_merge_kernel<DT, MET, VPL>, smem_merge) : e;
     }
     static cudaError_t occ(uint32_t threads, size_t smem, int *blocks)
     {

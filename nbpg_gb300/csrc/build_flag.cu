@@ -11,8 +11,7 @@ template <int DT, int MET, int VPL>
 static cudaError_t search_v(uint32_t grid, uint32_t warps, size_t smem, const BuildFlagArgs &F, int *blocks, cudaStream_t st)
 {
     if (blocks) {  // set-up: the shared memory this launch shape needs, and its residency
-        cudaError_t e = cudaFuncSetAttribute(build_search_kernel<DT, MET, VPL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             int(smem));
+        cudaError_t e = raise_smem_limit(build_search_kernel<DT, MET, VPL>, smem);
         if (e == cudaSuccess)
             e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, build_search_kernel<DT, MET, VPL>, int(warps * 32), smem);
         return e;
@@ -32,9 +31,7 @@ static cudaError_t search_t(uint32_t grid, uint32_t warps, size_t smem, const Bu
 template <int DT, int MET>
 static cudaError_t prune_t(uint32_t grid, const BuildFlagArgs &F, const PruneLayout &lay, cudaStream_t st)
 {
-    if (grid == 0)
-        return cudaFuncSetAttribute(build_prune_kernel<PRUNE_THREADS, DT, MET>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    int(lay.bytes));
+    if (grid == 0) return raise_smem_limit(build_prune_kernel<PRUNE_THREADS, DT, MET>, lay.bytes);
     build_prune_kernel<PRUNE_THREADS, DT, MET><<<grid, PRUNE_THREADS, lay.bytes, st>>>(F, lay);
     return cudaGetLastError();
 }

@@ -272,7 +272,7 @@ __global__ void __launch_bounds__(GT_THREADS) gt_kernel(GtArgs a)
 template <int DT, int MET>
 static cudaError_t launch_gt(const GtArgs &a, size_t smem, cudaStream_t st)
 {
-    cudaError_t e = cudaFuncSetAttribute(gt_kernel<DT, MET>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    cudaError_t e = raise_smem_limit(gt_kernel<DT, MET>, smem);
     if (e != cudaSuccess) return e;
     const uint32_t grid = (a.nq + GT_QT - 1) / GT_QT;
     gt_kernel<DT, MET><<<grid, GT_THREADS, smem, st>>>(a);

@@ -971,9 +971,9 @@ nbpg_status gt_scan_device(uint32_t dtype, uint32_t metric, uint32_t dims, uint3
     }
     const size_t smem = scan_smem(l.katoms, l.mt, ring ? ring : 2);
     if (e == cudaSuccess && s == NBPG_OK)
-        e = cudaFuncSetAttribute(gt_scan_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+        e = raise_smem_limit(gt_scan_kernel<true>, smem);
     if (e == cudaSuccess && s == NBPG_OK)
-        e = cudaFuncSetAttribute(gt_scan_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+        e = raise_smem_limit(gt_scan_kernel<false>, smem);
 
     ReplayArgs r{};
     r.s.bval = bval;

@@ -950,11 +950,9 @@ nbpg_status gt_tc_device(uint32_t dtype, uint32_t metric, uint32_t dims, uint32_
     const size_t smem = gt_tc_smem(l.katoms, k, stages ? stages : 2);
     const size_t msmem = gt_tc_merge_smem(k);
     if (e == cudaSuccess && s == NBPG_OK)
-        e = cudaFuncSetAttribute(metric == NBPG_L2 ? gt_tc_kernel<M_L2> : gt_tc_kernel<M_IP>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+        e = raise_smem_limit(metric == NBPG_L2 ? gt_tc_kernel<M_L2> : gt_tc_kernel<M_IP>, smem);
     if (e == cudaSuccess && s == NBPG_OK)
-        e = cudaFuncSetAttribute(metric == NBPG_L2 ? gt_tc_merge_kernel<M_L2> : gt_tc_merge_kernel<M_IP>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, int(msmem));
+        e = raise_smem_limit(metric == NBPG_L2 ? gt_tc_merge_kernel<M_L2> : gt_tc_merge_kernel<M_IP>, msmem);
     TcArgs a{};
     a.qnorm = qn;
     a.bnorm = bn;

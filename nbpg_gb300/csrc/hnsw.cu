@@ -50,15 +50,9 @@ template <int DT, int MET, int VPL>
 struct HnswKernels {
     static cudaError_t setup(size_t smem_level, size_t smem_merge, size_t smem_query)
     {
-        cudaError_t e = cudaFuncSetAttribute(hnsw_level_kernel<DT, MET, VPL>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem_level));
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(rev_merge_kernel<DT, MET, VPL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     int(smem_merge));
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(hnsw_descend_kernel<DT, MET, VPL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     int(smem_query));
-        return e;
+        cudaError_t e = raise_smem_limit(hnsw_level_kernel<DT, MET, VPL>, smem_level);
+        if (e == cudaSuccess) e = raise_smem_limit(rev_merge_kernel<DT, MET, VPL>, smem_merge);
+        return e == cudaSuccess ? raise_smem_limit(hnsw_descend_kernel<DT, MET, VPL>, smem_query) : e;
     }
     static cudaError_t occ_level(uint32_t threads, size_t smem, int *blocks)
     {

@@ -34,6 +34,15 @@ void set_error(const std::string &msg);
 
 inline uint32_t round_up(uint32_t x, uint32_t m) { return (x + m - 1) / m * m; }
 
+// Raises a kernel's dynamic shared-memory limit on the current device to at least `bytes`.  Never lowers it: the
+// limit belongs to the kernel, not to a call, and another thread may be about to launch with a larger layout.
+cudaError_t raise_smem_limit(const void *kernel, size_t bytes);
+template <class... A>
+inline cudaError_t raise_smem_limit(void (*kernel)(A...), size_t bytes)
+{
+    return raise_smem_limit(reinterpret_cast<const void *>(kernel), bytes);
+}
+
 // Growable device scratch buffer owned by an index.
 struct DevBuf {
     void *ptr = nullptr;

@@ -50,3 +50,27 @@ for i in range(3):
 idx.close()
 assert shim.shim_peak() > 0 and shim.shim_overrun() == 0
 """)
+
+
+def test_shared_memory_limits_are_never_lowered(shim):
+    """A kernel's limit belongs to every call of the process: one that needs less leaves it alone."""
+    shim("""
+def build(n, dims, R, L, VL, metric, fgim=False):
+    idx = Index(r.integers(0, 256, (n, dims)).astype(np.uint8), "u8", metric, max_degree=R)
+    (idx.build_fgim if fgim else idx.build_vamana)(L=L, VL=VL, num_split=2 if fgim else 0, num_passes=2 if fgim else 1)
+    idx.close()
+for dims, R, L, VL in [(256, 48, 90, 140), (64, 16, 24, 32), (256, 48, 90, 140)]:
+    for metric in ("l2", "ip"):
+        build(600, dims, R, L, VL, metric)
+    build(600, dims, R, L, VL, "l2", fgim=True)
+for dims, k in [(400, 100), (128, 100), (16, 1), (700, 150), (700, 3)]:
+    rows = r.integers(0, 256, (900, dims)).astype(np.uint8)
+    for engine in ("auto", "dp4a") + (("tensor",) if dims <= 128 else ()):
+        ground_truth(rows, rows[:40], "u8", "l2", k=k, engine=engine)
+for L in (90, 24):
+    idx = Index(r.integers(0, 256, (600, 64)).astype(np.uint8), "u8", "l2", max_degree=16)
+    h, _ = idx.build_hnsw(L=L, VL=190)
+    h.close()
+    idx.close()
+assert shim.shim_peak() > 0 and shim.shim_lowered() == 0
+""")
