@@ -314,10 +314,11 @@ nbpg_status nbpg_gt_with_engine(uint32_t dtype, uint32_t metric, uint32_t dims, 
  * nbpg_gt_workspace_size() bytes of device workspace (0 for DP4A); d_workspace NULL
  * makes the call allocate it.  The size depends on the current device's SM count: the
  * tensor engine cuts the scans into one range per SM and keeps, per range and query, a list
- * of up to 4,096 candidates (1.6 GB on 152 SMs for 10k queries at k = 100, besides the bf16
- * copies of base and queries).  With AUTO, rows or k past the TENSOR limits also run where the
- * workspace is smaller than that or cannot be allocated (the call allocates its own, or takes
- * DP4A).  Returns after the work has finished on `stream`. */
+ * of up to 512 to 4,096 candidates (10k queries on 1M rows of 128 codes, 152 SMs: 1.5 GB at
+ * k = 100 and 0.6 GB at k = 10, of which 0.26 GB are the bf16 copy of the base).  With AUTO, rows
+ * or k past the TENSOR limits also run where the workspace is smaller than that (the call
+ * allocates its own), and a call whose workspace cannot be allocated takes DP4A, which needs none.
+ * Returns after the work has finished on `stream`. */
 nbpg_status nbpg_gt_workspace_size(uint32_t dtype, uint32_t dims, uint64_t n, uint32_t nq, uint32_t k,
                                    uint32_t engine, size_t *bytes);
 nbpg_status nbpg_gt_device(uint32_t dtype, uint32_t metric, uint32_t dims, uint32_t row_stride, const void *d_base,

@@ -283,12 +283,12 @@ bool gt_tc_supported(uint32_t dtype, uint32_t dims, uint32_t k, size_t smem_opti
 nbpg_status gt_tc_device(uint32_t dtype, uint32_t metric, uint32_t dims, uint32_t stride, const uint8_t *d_base,
                          uint64_t n, const uint8_t *d_q, uint32_t nq, uint32_t k, uint32_t mode, uint32_t *d_ids,
                          float *d_dists, void *ws, cudaStream_t st);
-size_t gt_tc_workspace(uint32_t dtype, uint32_t dims, uint64_t n, uint32_t nq, uint32_t k);
+size_t gt_tc_workspace(uint32_t dtype, uint32_t dims, uint64_t n, uint32_t nq, uint32_t k, uint32_t sms = 0);
 bool gt_scan_supported(uint32_t dtype, uint32_t dims, uint32_t k, size_t smem_optin);
 nbpg_status gt_scan_device(uint32_t dtype, uint32_t metric, uint32_t dims, uint32_t stride, const uint8_t *d_base,
                            uint64_t n, const uint8_t *d_q, uint32_t nq, uint32_t k, uint32_t mode, uint32_t *d_ids,
                            float *d_dists, void *ws, cudaStream_t st, bool *overflow, bool withhold = false);
-size_t gt_scan_workspace(uint32_t dtype, uint32_t dims, uint64_t n, uint32_t nq, uint32_t k);
+size_t gt_scan_workspace(uint32_t dtype, uint32_t dims, uint64_t n, uint32_t nq, uint32_t k, uint32_t sms = 0);
 
 nbpg_status gt_device(uint32_t dtype, uint32_t metric, const GtArgs &a, cudaStream_t st, size_t smem_optin)
 {
@@ -324,6 +324,7 @@ using namespace nbpg;
 struct GtPlan {
     bool scan;    // the staged scan
     bool replay;  // the replaying tensor engine takes this shape (rows of up to 128 codes, k <= 100)
+    bool dp4a;    // the call did not ask for the tensor cores
     size_t smem_optin;
 };
 
@@ -336,6 +337,7 @@ static nbpg_status resolve_engine(uint32_t dtype, uint32_t dims, uint32_t k, uin
     out->smem_optin = size_t(optin);
     out->replay = gt_tc_supported(dtype, dims, k, size_t(optin));
     out->scan = engine != NBPG_GT_DP4A && gt_scan_supported(dtype, dims, k, size_t(optin));
+    out->dp4a = engine != NBPG_GT_TENSOR;
     if (engine == NBPG_GT_TENSOR && !(out->replay && out->scan)) {
         set_error("nbpg_gt: the tensor engine needs <= 128 codes per row and k <= 100");
         return NBPG_ERR_UNSUPPORTED;
@@ -351,8 +353,8 @@ static size_t plan_workspace(const GtPlan &p, uint32_t dtype, uint32_t dims, uin
 }
 
 // Runs the plan; returns when the work is done or, for DP4A, enqueued.  ws holds plan_workspace()
-// bytes, or is NULL: the tensor engines then allocate theirs, and where DP4A alone used to run
-// (longer rows, larger k) it still does if that memory is not to be had.
+// bytes, or is NULL: the tensor engines then allocate theirs, and where that memory is not to be had the
+// next one in line runs, in the end DP4A, which needs none (unless the call asked for the tensor cores).
 static nbpg_status run_plan(const GtPlan &p, uint32_t dtype, uint32_t metric, uint32_t dims, const GtArgs &a, uint32_t mode,
                             void *ws, cudaStream_t st)
 {
@@ -360,11 +362,12 @@ static nbpg_status run_plan(const GtPlan &p, uint32_t dtype, uint32_t metric, ui
         bool overflow = false;
         const nbpg_status s = gt_scan_device(dtype, metric, dims, a.row_stride, a.base, a.n, a.queries, a.nq, a.k, mode,
                                              a.out_ids, a.out_dists, ws, st, &overflow);
-        if (s == NBPG_OK && !overflow) return s;
-        if (s != NBPG_OK && !(s == NBPG_ERR_OOM && !p.replay)) return s;
-        if (p.replay)
-            return gt_tc_device(dtype, metric, dims, a.row_stride, a.base, a.n, a.queries, a.nq, a.k, mode, a.out_ids,
-                                a.out_dists, ws, st);
+        if (s != NBPG_OK ? s != NBPG_ERR_OOM : !overflow) return s;
+        if (p.replay) {
+            const nbpg_status r = gt_tc_device(dtype, metric, dims, a.row_stride, a.base, a.n, a.queries, a.nq, a.k, mode,
+                                               a.out_ids, a.out_dists, ws, st);
+            if (r != NBPG_ERR_OOM || !p.dp4a) return r;
+        }
     }
     return gt_device(dtype, metric, a, st, p.smem_optin);
 }
@@ -469,4 +472,14 @@ extern "C" nbpg_status nbpg_gt_device(uint32_t dtype, uint32_t metric, uint32_t 
     s = run_plan(plan, dtype, metric, dims, a, mode, workspace_bytes >= need ? d_workspace : nullptr, st);
     if (s == NBPG_OK) NBPG_CUDA_TRY(cudaStreamSynchronize(st));
     return s;
+}
+
+// Test hook: the workspaces of the staged scan and of the replaying engine on a device of `sms` SMs (host code only)
+extern "C" nbpg_status nbpg_test_gt_workspace(uint32_t dtype, uint32_t dims, uint64_t n, uint32_t nq, uint32_t k, uint32_t sms,
+                                              size_t *scan, size_t *replay)
+{
+    NBPG_CHECK_ARG(scan && replay && n >= 1 && nq >= 1 && k >= 1 && sms >= 1, "bad argument");
+    *scan = gt_scan_workspace(dtype, dims, n, nq, k, sms);
+    *replay = gt_tc_workspace(dtype, dims, n, nq, k, sms);
+    return NBPG_OK;
 }

@@ -39,7 +39,8 @@ constexpr uint32_t SC_SLOTS = 4;         // TMEM accumulators of 128 columns: al
 constexpr uint32_t SC_MAX_STAGES = 8;    // shared-memory ring of base chunks (1 or 2 columns of 64 codes each)
 constexpr int SC_THREADS = 352;          // warps 0-7 epilogue (4 per query tile of 128), 8 TMA, 9 MMA, 10 base values
 constexpr uint32_t SC_P0 = 8;            // base tiles of the first stage
-constexpr uint32_t SC_CAP = 4096;        // most records of one query in one range
+constexpr uint32_t SC_CAP = 4096;        // most records of one query in one range (fewer where memory says so)
+constexpr uint32_t SC_CAP_MIN = 512;
 constexpr uint32_t SC_BATCH = 64;        // query tiles per batch (up to 16,384 queries)
 constexpr uint32_t SC_MAX_K = 128;
 constexpr uint32_t SC_MAX_ELEMS = 640;
@@ -59,9 +60,9 @@ struct ScanArgs {
     uint64_t W, total;   // steps per range, and in all
     uint32_t stages, withhold;
     const float *bound;  // per query: B
-    uint2 *lists;        // [range + query tile][query of the tile][cap] (ordered distance, id)
+    uint2 *lists;        // [range + query tile][query of the tile, lrows of them][cap] (ordered distance, id)
     uint32_t *list_n;    // [range + query tile][query of the tile]
-    uint32_t cap;
+    uint32_t cap, lrows;
     float *dense;        // first stage: [query][dense_stride] distances
     uint32_t dense_stride;
     uint32_t *err;
@@ -408,11 +409,11 @@ __global__ void __launch_bounds__(SC_THREADS, 1)
             const uint32_t q = li * qrows + row;
             const bool live = q < a.nq;
             const float qv = live ? a.qval[q] : 0.0f;
-            const size_t sidx = (size_t(blockIdx.x) + li) * qrows + row;
+            const size_t sidx = (size_t(blockIdx.x) + li) * a.lrows + row;  // (of live queries: row < lrows)
             ScanRow sr{-kInf, -kInf, qv, c2, nullptr, 0u};
             if constexpr (!DENSE) {
-                sr.lst = a.lists + sidx * a.cap;
                 if (live) {
+                    sr.lst = a.lists + sidx * a.cap;
                     sr.B = a.bound[q];
                     sr.thr = __fadd_ru(__fsub_ru(__fdiv_rn(sr.B, float(a.scale)), qv), a.slack);
                 }
@@ -457,7 +458,8 @@ __global__ void __launch_bounds__(SC_THREADS, 1)
                 mbar_arrive(bar_tempty + 8 * slot);
                 // (with two query tiles the base values are released by both tiles' accumulators)
             }
-            if constexpr (!DENSE) a.list_n[sidx] = sr.ln;
+            if constexpr (!DENSE)
+                if (live) a.list_n[sidx] = sr.ln;
             p += b1 - b0;
         }
     }
@@ -654,7 +656,7 @@ __global__ void __launch_bounds__(128) gt_replay_kernel(ReplayArgs a)
         const uint32_t c0 = uint32_t(li * T / a.s.W), c1 = uint32_t(((li + 1) * T - 1) / a.s.W);
         for (uint32_t s0 = c0; s0 <= c1; s0 += 32) {
             const uint32_t c = s0 + lane;
-            uint32_t cnt = c <= c1 ? a.s.list_n[size_t(c + li) * qrows + row] : 0u;
+            uint32_t cnt = c <= c1 ? a.s.list_n[size_t(c + li) * a.s.lrows + row] : 0u;
             if (__any_sync(kFull, cnt > a.s.cap)) {
                 if (lane == 0) atomicExch(a.ovf, 1u);  // records lost: the host takes another engine
                 cnt = min(cnt, a.s.cap);
@@ -677,7 +679,7 @@ __global__ void __launch_bounds__(128) gt_replay_kernel(ReplayArgs a)
                 j = min(j, 31u);
                 const uint32_t off = e - __shfl_sync(kFull, excl, int(j));
                 uint2 rec = make_uint2(0u, 0u);
-                if (e < all) rec = a.s.lists[(size_t(s0 + j + li) * qrows + row) * a.s.cap + off];
+                if (e < all) rec = a.s.lists[(size_t(s0 + j + li) * a.s.lrows + row) * a.s.cap + off];
                 if constexpr (EXACT) ex_batch(ex, buf, k, rec.x, rec.y, e < all, lane);
                 else cg_batch(cg, rec.x, rec.y, e < all, lane);
             }
@@ -829,19 +831,34 @@ struct ScanSplit {
     uint32_t ctas, cap;
 };
 
-// One equal range of steps per SM; a range holds at most `cap` records per query.
-static ScanSplit scan_split(uint32_t qtiles, uint32_t T, uint32_t sms)
+// One equal range of steps per SM; a range holds at most `most` records per query.
+static ScanSplit scan_split(uint32_t qtiles, uint32_t T, uint32_t sms, uint32_t most)
 {
     ScanSplit s;
     s.total = uint64_t(qtiles) * T;
     s.W = (s.total + sms - 1) / sms;
     s.ctas = uint32_t((s.total + s.W - 1) / s.W);
-    s.cap = uint32_t(std::min<uint64_t>(SC_CAP, std::min<uint64_t>(s.W, T) * SC_ROWS));
+    s.cap = uint32_t(std::min<uint64_t>(most, std::min<uint64_t>(s.W, T) * SC_ROWS));
     return s;
+}
+
+size_t gt_tc_list_bytes(uint64_t n, uint32_t nq, uint32_t k, uint32_t sms);
+
+// Most records of one query in one range.  A stage records about 3 k rows of a query (15 k where k is small) over all
+// its ranges, two at least, so what the lists have past SC_CAP_MIN is room for rows in an order.  That room is given
+// within the memory that the replaying engine takes for its lists (up to 0.32, 0.64 or 1.27 GB for k up to 25, 51 and
+// above, on 152 SMs), less `other`, the rest of this scan's state.  Lists are kept for live queries only.
+static uint32_t scan_most(uint64_t n, uint32_t nq, uint32_t k, uint32_t sms, uint32_t batch, uint32_t lrows, size_t other)
+{
+    const size_t room = gt_tc_list_bytes(n, nq, k, sms);
+    const size_t per = size_t(sms + batch) * lrows * 8;
+    const size_t fit = room > other ? (room - other) / per / SC_ROWS * SC_ROWS : 0;
+    return uint32_t(std::min<size_t>(SC_CAP, std::max<size_t>(SC_CAP_MIN, fit)));
 }
 
 struct ScanLayout {
     uint32_t K, katoms, mt, qrows, batch;  // batch: query tiles per pass
+    uint32_t lrows, most;                  // queries of a tile that lists are kept for; their longest
     uint64_t n_pad, nq_pad;
     std::vector<uint32_t> at;
     size_t off_q, off_bval, off_qval, off_flags, off_bound, off_d, off_i, off_top, off_dense, off_listn, off_lists, bytes;
@@ -858,15 +875,19 @@ static ScanLayout scan_layout(uint32_t dtype, uint32_t dims, uint64_t n, uint32_
     l.nq_pad = (uint64_t(nq) + l.qrows - 1) / l.qrows * l.qrows;
     l.at = scan_stages(uint32_t(l.n_pad / SC_ROWS), k);
     l.batch = uint32_t(std::min<uint64_t>(SC_BATCH, l.nq_pad / l.qrows));
-    size_t lists = 0, segs = 0;
-    for (size_t i = 1; i + 1 < l.at.size(); ++i) {
-        const ScanSplit s = scan_split(l.batch, l.at[i + 1] - l.at[i], sms);
-        // a smaller last batch has shorter ranges, and up to one per SM of them
-        lists = std::max(lists, size_t(sms + l.batch) * l.qrows * s.cap);
-        segs = std::max(segs, size_t(sms + l.batch) * l.qrows);
-    }
-    const size_t qb = size_t(l.batch) * l.qrows;
+    l.lrows = uint32_t(std::min<uint64_t>(nq, l.qrows));
     auto up = [](size_t x) { return (x + 255) / 256 * 256; };
+    const size_t qb = std::min<size_t>(nq, size_t(l.batch) * l.qrows);
+    l.most = scan_most(n, nq, k, sms, l.batch, l.lrows, qb * (l.at[1] * SC_ROWS * 4 + 1036));
+    size_t lists = 0, segs = 0;
+    const uint64_t qtiles = l.nq_pad / l.qrows;
+    for (size_t i = 1; i + 1 < l.at.size(); ++i)
+        for (uint64_t qt : {uint64_t(l.batch), qtiles % l.batch})  // a full batch and the last one
+            if (qt) {
+                const ScanSplit s = scan_split(uint32_t(qt), l.at[i + 1] - l.at[i], sms, l.most);
+                lists = std::max(lists, size_t(s.ctas + qt) * l.lrows * s.cap);
+                segs = std::max(segs, size_t(s.ctas + qt) * l.lrows);
+            }
     l.off_q = up(l.n_pad * l.K * 2);
     l.off_bval = l.off_q + up(l.nq_pad * l.K * 2);
     l.off_qval = l.off_bval + up(l.n_pad * 4);
@@ -891,9 +912,10 @@ static uint32_t scan_sms()
     return uint32_t(sms);
 }
 
-size_t gt_scan_workspace(uint32_t dtype, uint32_t dims, uint64_t n, uint32_t nq, uint32_t k)
+// sms 0: the current device's
+size_t gt_scan_workspace(uint32_t dtype, uint32_t dims, uint64_t n, uint32_t nq, uint32_t k, uint32_t sms)
 {
-    return scan_layout(dtype, dims, n, nq, k, scan_sms()).bytes;
+    return scan_layout(dtype, dims, n, nq, k, sms ? sms : scan_sms()).bytes;
 }
 
 template <int DT>
@@ -916,7 +938,7 @@ static void launch_replay(uint32_t metric, const ReplayArgs &r, cudaStream_t st)
 // Device-resident inputs (rows of dims bytes, stride bytes apart); outputs device arrays nq * k.
 // ws: gt_scan_workspace() bytes, or NULL to allocate them here.  Returns after the work has finished
 // on `st`.  *overflow is set when a record list was too short (rows that come closer and closer to
-// a query, more than 4,096 of them in one range): the outputs are then incomplete and the caller
+// a query, more of them in one range than a list holds): the outputs are then incomplete and the caller
 // takes an engine without lists.
 nbpg_status gt_scan_device(uint32_t dtype, uint32_t metric, uint32_t dims, uint32_t stride, const uint8_t *d_base,
                            uint64_t n, const uint8_t *d_q, uint32_t nq, uint32_t k, uint32_t mode, uint32_t *d_ids,
@@ -993,6 +1015,7 @@ nbpg_status gt_scan_device(uint32_t dtype, uint32_t metric, uint32_t dims, uint3
     r.s.list_n = reinterpret_cast<uint32_t *>(w + l.off_listn);
     r.s.dense = reinterpret_cast<float *>(w + l.off_dense);
     r.s.dense_stride = l.at[1] * SC_ROWS;
+    r.s.lrows = l.lrows;
     r.s.err = flags;
     r.k = k;
     r.st_d = reinterpret_cast<uint4 *>(w + l.off_d);
@@ -1010,7 +1033,7 @@ nbpg_status gt_scan_device(uint32_t dtype, uint32_t metric, uint32_t dims, uint3
         for (size_t i = 0; i + 1 < l.at.size(); ++i) {
             r.s.b_first = l.at[i];
             r.s.T = l.at[i + 1] - l.at[i];
-            const ScanSplit sp = scan_split(qtiles, r.s.T, sms);
+            const ScanSplit sp = scan_split(qtiles, r.s.T, sms, l.most);
             r.s.W = sp.W;
             r.s.total = sp.total;
             r.s.cap = sp.cap;

@@ -878,9 +878,17 @@ static TcLayout tc_layout(uint32_t dtype, uint32_t dims, uint64_t n, uint32_t nq
     return l;
 }
 
-size_t gt_tc_workspace(uint32_t dtype, uint32_t dims, uint64_t n, uint32_t nq, uint32_t k)
+// Memory of the continuation lists alone
+size_t gt_tc_list_bytes(uint64_t n, uint32_t nq, uint32_t k, uint32_t sms)
 {
-    return tc_layout(dtype, dims, n, nq, k, device_sms()).bytes;
+    const TcSplit sp = tc_split((uint64_t(nq) + TC_M - 1) / TC_M, (n + TC_N - 1) / TC_N, k, sms);
+    return size_t(sp.ctas) * TC_M * sp.cap * 8;
+}
+
+// sms 0: the current device's
+size_t gt_tc_workspace(uint32_t dtype, uint32_t dims, uint64_t n, uint32_t nq, uint32_t k, uint32_t sms)
+{
+    return tc_layout(dtype, dims, n, nq, k, sms ? sms : device_sms()).bytes;
 }
 
 // Device-resident inputs (rows of dims bytes, stride bytes apart); outputs device arrays
@@ -899,6 +907,7 @@ nbpg_status gt_tc_device(uint32_t dtype, uint32_t metric, uint32_t dims, uint32_
     if (!ws) {
         e = cudaMalloc(&owned, l.bytes);
         if (e != cudaSuccess) {
+            cudaGetLastError();  // an allocation that did not fit is not a fault of later launches
             set_error(std::string("nbpg_gt (tensor path): ") + cudaGetErrorString(e));
             return e == cudaErrorMemoryAllocation ? NBPG_ERR_OOM : NBPG_ERR_CUDA;
         }

@@ -74,3 +74,26 @@ for L in (90, 24):
     idx.close()
 assert shim.shim_peak() > 0 and shim.shim_lowered() == 0
 """)
+
+
+def test_knn_runs_in_the_memory_it_has(shim):
+    """One query over 200k rows within the rows' own copies and 64 MB; with no room for any list, AUTO runs on DP4A
+    and the explicit tensor engine says so."""
+    shim("""
+base = r.integers(0, 256, (200000, 128)).astype(np.uint8)
+want = ground_truth(base, base[:1], "u8", "l2", k=100, engine="dp4a")
+shim.shim_limit(base.nbytes * 3 + (64 << 20))
+got = ground_truth(base, base[:1], "u8", "l2", k=100, engine="tensor")
+assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
+shim.shim_limit(base.nbytes + (1 << 20))
+got = ground_truth(base, base[:1], "u8", "l2", k=100)
+assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
+try:
+    ground_truth(base, base[:1], "u8", "l2", k=100, engine="tensor")
+    raise SystemExit("no refusal")
+except _lib.NbpgError as e:
+    assert e.status == 2
+shim.shim_limit(1 << 40)
+got = ground_truth(base, base[:1], "u8", "l2", k=100)
+assert np.array_equal(got[0], want[0]) and shim.shim_overrun() == 0 and shim.shim_peak() > 0
+""")
