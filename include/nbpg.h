@@ -314,8 +314,8 @@ nbpg_status nbpg_gt_with_engine(uint32_t dtype, uint32_t metric, uint32_t dims, 
  * nbpg_gt_workspace_size() bytes of device workspace (0 for DP4A); d_workspace NULL
  * makes the call allocate it.  The size depends on the current device's SM count: the
  * tensor engine cuts the scans into one range per SM and keeps, per range and query, a list
- * of up to 512 to 4,096 candidates (10k queries on 1M rows of 128 codes, 152 SMs: 1.5 GB at
- * k = 100 and 0.6 GB at k = 10, of which 0.26 GB are the bf16 copy of the base).  With AUTO, rows
+ * of candidates that can grow from a shared pool (10k queries on 1M rows of 128 codes, 152 SMs:
+ * 1.5 GB at k = 100 and 0.6 GB at k = 10, of which 0.26 GB are the bf16 copy of the base).  With AUTO, rows
  * or k past the TENSOR limits also run where the workspace is smaller than that (the call
  * allocates its own), and a call whose workspace cannot be allocated takes DP4A, which needs none.
  * Returns after the work has finished on `stream`. */

@@ -92,6 +92,8 @@ def lib() -> C.CDLL:
                               C.c_uint32, _u32p, _f32p, _u32p, _u32p, _u32p]
     L.nbpg_search_device.argtypes = [_vp, _vp, C.c_uint32, C.POINTER(SearchParams), _vp, _vp, _u32p, C.c_uint32,
                                      C.c_uint32, _vp, _vp, _vp, _vp, _vp, _vp]
+    L.nbpg_test_gt_redone.argtypes = [C.c_uint32, C.c_uint32, C.c_uint32, _vp, C.c_uint64, _vp, C.c_uint32, C.c_uint32,
+                                      C.c_uint32, _u32p, _f32p, C.c_int32, C.c_uint32, _u32p]
     L.nbpg_test_gt_workspace.argtypes = [C.c_uint32, C.c_uint32, C.c_uint64, C.c_uint32, C.c_uint32, C.c_uint32,
                                          C.POINTER(C.c_size_t), C.POINTER(C.c_size_t)]
     L.nbpg_test_gt_split.argtypes = [C.c_uint32, C.c_uint32, C.c_uint32, C.c_uint32, _u32p,

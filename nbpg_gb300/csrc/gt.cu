@@ -287,7 +287,8 @@ size_t gt_tc_workspace(uint32_t dtype, uint32_t dims, uint64_t n, uint32_t nq, u
 bool gt_scan_supported(uint32_t dtype, uint32_t dims, uint32_t k, size_t smem_optin);
 nbpg_status gt_scan_device(uint32_t dtype, uint32_t metric, uint32_t dims, uint32_t stride, const uint8_t *d_base,
                            uint64_t n, const uint8_t *d_q, uint32_t nq, uint32_t k, uint32_t mode, uint32_t *d_ids,
-                           float *d_dists, void *ws, cudaStream_t st, bool *overflow, bool withhold = false);
+                           float *d_dists, void *ws, cudaStream_t st, uint32_t *redone, uint32_t most_blocks,
+                           bool withhold = false);
 size_t gt_scan_workspace(uint32_t dtype, uint32_t dims, uint64_t n, uint32_t nq, uint32_t k, uint32_t sms = 0);
 
 nbpg_status gt_device(uint32_t dtype, uint32_t metric, const GtArgs &a, cudaStream_t st, size_t smem_optin)
@@ -319,8 +320,8 @@ nbpg_status gt_device(uint32_t dtype, uint32_t metric, const GtArgs &a, cudaStre
 
 using namespace nbpg;
 
-// What a call runs: the staged tensor scan (gt_scan.cu), with the replaying tensor engine (gt_tc.cu)
-// behind it for record lists that overflow, or DP4A.
+// What a call runs: the staged tensor scan (gt_scan.cu); where its memory is not to be had, the replaying
+// tensor engine (gt_tc.cu), which needs less of it at some sizes; or DP4A.
 struct GtPlan {
     bool scan;    // the staged scan
     bool replay;  // the replaying tensor engine takes this shape (rows of up to 128 codes, k <= 100)
@@ -356,13 +357,12 @@ static size_t plan_workspace(const GtPlan &p, uint32_t dtype, uint32_t dims, uin
 // bytes, or is NULL: the tensor engines then allocate theirs, and where that memory is not to be had the
 // next one in line runs, in the end DP4A, which needs none (unless the call asked for the tensor cores).
 static nbpg_status run_plan(const GtPlan &p, uint32_t dtype, uint32_t metric, uint32_t dims, const GtArgs &a, uint32_t mode,
-                            void *ws, cudaStream_t st)
+                            void *ws, cudaStream_t st, uint32_t *redone = nullptr, uint32_t most_blocks = ~0u)
 {
     if (p.scan) {
-        bool overflow = false;
         const nbpg_status s = gt_scan_device(dtype, metric, dims, a.row_stride, a.base, a.n, a.queries, a.nq, a.k, mode,
-                                             a.out_ids, a.out_dists, ws, st, &overflow);
-        if (s != NBPG_OK ? s != NBPG_ERR_OOM : !overflow) return s;
+                                             a.out_ids, a.out_dists, ws, st, redone, most_blocks);
+        if (s != NBPG_ERR_OOM) return s;
         if (p.replay) {
             const nbpg_status r = gt_tc_device(dtype, metric, dims, a.row_stride, a.base, a.n, a.queries, a.nq, a.k, mode,
                                                a.out_ids, a.out_dists, ws, st);
@@ -380,9 +380,9 @@ extern "C" nbpg_status nbpg_gt(uint32_t dtype, uint32_t metric, uint32_t dims, c
                                device);
 }
 
-extern "C" nbpg_status nbpg_gt_with_engine(uint32_t dtype, uint32_t metric, uint32_t dims, const void *base,
-                                           uint64_t n, const void *queries, uint32_t nq, uint32_t k, uint32_t mode,
-                                           uint32_t engine, uint32_t *out_ids, float *out_dists, int32_t device)
+static nbpg_status gt_host(uint32_t dtype, uint32_t metric, uint32_t dims, const void *base, uint64_t n, const void *queries,
+                           uint32_t nq, uint32_t k, uint32_t mode, uint32_t engine, uint32_t *out_ids, float *out_dists,
+                           int32_t device, uint32_t *redone = nullptr, uint32_t most_blocks = ~0u)
 {
     NBPG_CHECK_ARG(base && queries && out_ids && out_dists, "null argument");
     NBPG_CHECK_ARG(dtype <= NBPG_I4 && metric <= NBPG_IP, "unsupported dtype/metric");
@@ -417,7 +417,7 @@ extern "C" nbpg_status nbpg_gt_with_engine(uint32_t dtype, uint32_t metric, uint
     if (s == NBPG_OK) s = resolve_engine(dtype, dims, k, engine, &plan);
     if (s == NBPG_OK) {
         const GtArgs a{db, n, rs, dq, nq, k, mode == NBPG_GT_EXACT ? 1u : 0u, di, dd};
-        s = run_plan(plan, dtype, metric, dims, a, mode, nullptr, st);
+        s = run_plan(plan, dtype, metric, dims, a, mode, nullptr, st, redone, most_blocks);
     }
     if (s == NBPG_OK) {
         e = cudaMemcpyAsync(out_ids, di, size_t(nq) * k * 4, cudaMemcpyDeviceToHost, st);
@@ -432,6 +432,21 @@ extern "C" nbpg_status nbpg_gt_with_engine(uint32_t dtype, uint32_t metric, uint
     cudaFree(dd);
     cudaStreamDestroy(st);
     return s;
+}
+
+extern "C" nbpg_status nbpg_gt_with_engine(uint32_t dtype, uint32_t metric, uint32_t dims, const void *base,
+                                           uint64_t n, const void *queries, uint32_t nq, uint32_t k, uint32_t mode,
+                                           uint32_t engine, uint32_t *out_ids, float *out_dists, int32_t device)
+{
+    return gt_host(dtype, metric, dims, base, n, queries, nq, k, mode, engine, out_ids, out_dists, device);
+}
+
+// Test hook: nbpg_gt with at most that many further blocks for record lists, and how many queries were scanned again
+extern "C" nbpg_status nbpg_test_gt_redone(uint32_t dtype, uint32_t metric, uint32_t dims, const void *base, uint64_t n,
+                                           const void *queries, uint32_t nq, uint32_t k, uint32_t mode, uint32_t *out_ids,
+                                           float *out_dists, int32_t device, uint32_t most_blocks, uint32_t *redone)
+{
+    return gt_host(dtype, metric, dims, base, n, queries, nq, k, mode, NBPG_GT_AUTO, out_ids, out_dists, device, redone, most_blocks);
 }
 
 extern "C" nbpg_status nbpg_gt_workspace_size(uint32_t dtype, uint32_t dims, uint64_t n, uint32_t nq, uint32_t k,

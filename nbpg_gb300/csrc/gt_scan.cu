@@ -8,7 +8,8 @@
 // one records, per query, the rows below the bound that the stage before left, about 3 k of them in
 // random order however long the stage; after each stage one warp per query replays its records in
 // id order and publishes the new bound.  Within a stage nothing waits on anything: the (query tile,
-// base tile) steps are cut into one equal range per SM.
+// base tile) steps are cut into one equal range per SM.  Queries for which rows stored in some order
+// fill a list are scanned again in stages too short for that (gt_scan_device).
 //
 // Against a scan that replays as it goes this takes the flagged candidates from 94% of the 32 x 32
 // chunks to about a third, and the sequential replay out of the scan altogether.
@@ -39,8 +40,10 @@ constexpr uint32_t SC_SLOTS = 4;         // TMEM accumulators of 128 columns: al
 constexpr uint32_t SC_MAX_STAGES = 8;    // shared-memory ring of base chunks (1 or 2 columns of 64 codes each)
 constexpr int SC_THREADS = 352;          // warps 0-7 epilogue (4 per query tile of 128), 8 TMA, 9 MMA, 10 base values
 constexpr uint32_t SC_P0 = 8;            // base tiles of the first stage
-constexpr uint32_t SC_CAP = 4096;        // most records of one query in one range (fewer where memory says so)
-constexpr uint32_t SC_CAP_MIN = 512;
+constexpr uint32_t SC_FIRST = 384;       // records in the first block of a list (one list per query and range)
+constexpr uint32_t SC_BLOCK = 512;       // records in each further block, from a pool that all lists share
+constexpr uint32_t SC_MORE = 31;         // most further blocks of a list
+constexpr uint32_t SC_LOST = ~0u;        // length of a list that found no block
 constexpr uint32_t SC_BATCH = 64;        // query tiles per batch (up to 16,384 queries)
 constexpr uint32_t SC_MAX_K = 128;
 constexpr uint32_t SC_MAX_ELEMS = 640;
@@ -63,6 +66,10 @@ struct ScanArgs {
     uint2 *lists;        // [range + query tile][query of the tile, lrows of them][cap] (ordered distance, id)
     uint32_t *list_n;    // [range + query tile][query of the tile]
     uint32_t cap, lrows;
+    uint2 *pool;         // [pool_blocks][SC_BLOCK] records past the first cap of a list
+    uint32_t *more;      // [range + query tile][query of the tile][SC_MORE] their blocks
+    uint32_t *pool_next;
+    uint32_t pool_blocks;
     float *dense;        // first stage: [query][dense_stride] distances
     uint32_t dense_stride;
     uint32_t *err;
@@ -71,10 +78,12 @@ struct ScanArgs {
 struct ReplayArgs {
     ScanArgs s;
     uint32_t k, first, last;
+    const uint32_t *rows;  // output row of each query, or null: its own
     uint4 *st_d, *st_i;  // [query][32 lanes] distances (ordered) and ids of the running list
     uint2 *st_top;       // [query] CompGT's topdist and toppos
     float *bound;
-    uint32_t *ovf;       // a record list overflowed
+    uint32_t *ovf;       // per query: a record list overflowed; null: that cannot be
+    uint32_t *any_ovf;
     uint32_t *out_ids;
     float *out_dists;
 };
@@ -154,7 +163,8 @@ struct ScanRow {
     float thr, B, qv;  // flag below thr; record below B; the query's value
     uint64_t c2;       // (c, c)
     uint2 *lst;
-    uint32_t ln;       // records so far (past the cap: counted only)
+    uint32_t ln, end;  // records so far, and how many the list has room for (lst[ln] is the next place)
+    uint32_t list;
 };
 
 // v[j] for a j known only at run time, by a tree of selects (the chunk stays in registers)
@@ -170,6 +180,25 @@ __device__ __forceinline__ uint32_t pick32(const uint32_t (&v)[32], uint32_t j)
 #pragma unroll
     for (int i = 0; i < 2; ++i) d[i] = (j & 2) ? c[i + 2] : c[i];
     return (j & 1) ? d[1] : d[0];
+}
+
+// A further block for a list that has no room for another base tile; the rest of the present one is filled with records
+// that no rule admits.  Without a block the query's records are lost (it is scanned for again later on), and nothing more
+// is recorded for it in this range.  Looked at once per tile, so that the record loop itself has no limit to check
+// (checked there it cost 12%: 10k x 1M, k = 100 in 4.80 ms instead of 4.21).
+__device__ __forceinline__ void scan_more(const ScanArgs &a, ScanRow &row)
+{
+    const uint32_t x = (row.end - a.cap) / SC_BLOCK;
+    const uint32_t b = x < SC_MORE && a.pool_blocks ? atomicAdd(a.pool_next, 1u) : a.pool_blocks;
+    if (b < a.pool_blocks) {
+        for (; row.ln < row.end; ++row.ln) row.lst[row.ln] = make_uint2(~0u, ~0u);
+        a.more[size_t(row.list) * SC_MORE + x] = b;
+        row.lst = a.pool + size_t(b) * SC_BLOCK - row.end;
+        row.end += SC_BLOCK;
+    } else {
+        row.thr = row.B = -__int_as_float(0x7f800000);
+        row.ln = SC_LOST;
+    }
 }
 
 // One thread's query row of an accumulator chunk: 32 dot products v, the base rows' values bn (in
@@ -214,10 +243,7 @@ __device__ __forceinline__ void scan_chunk(const ScanArgs &a, const uint32_t (&v
         mask &= mask - 1;
         const int32_t dot = __float2int_rn(__uint_as_float(pick32(v, e)));
         const float df = __int2float_rn((__float2int_rn(row.qv) + __float2int_rn(bn[e]) + a.c * dot) * a.scale);
-        if (df < row.B) {
-            if (row.ln < a.cap) row.lst[row.ln] = make_uint2(f2ord(df), id0 + e);
-            ++row.ln;
-        }
+        if (df < row.B) row.lst[row.ln++] = make_uint2(f2ord(df), id0 + e);
     }
 }
 
@@ -410,7 +436,7 @@ __global__ void __launch_bounds__(SC_THREADS, 1)
             const bool live = q < a.nq;
             const float qv = live ? a.qval[q] : 0.0f;
             const size_t sidx = (size_t(blockIdx.x) + li) * a.lrows + row;  // (of live queries: row < lrows)
-            ScanRow sr{-kInf, -kInf, qv, c2, nullptr, 0u};
+            ScanRow sr{-kInf, -kInf, qv, c2, nullptr, 0u, a.cap, uint32_t(sidx)};
             if constexpr (!DENSE) {
                 if (live) {
                     sr.lst = a.lists + sidx * a.cap;
@@ -427,6 +453,8 @@ __global__ void __launch_bounds__(SC_THREADS, 1)
                     break;
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                if constexpr (!DENSE)
+                    if (sr.end - sr.ln < SC_ROWS) scan_more(a, sr);
                 const float *bn = nring + ns * SC_ROWS;
                 const uint32_t ta = tmem + tlane + slot * SC_ROWS;
                 const uint32_t id0 = (a.b_first + b) * SC_ROWS;
@@ -597,7 +625,9 @@ __global__ void __launch_bounds__(128) gt_replay_kernel(ReplayArgs a)
     __shared__ uint64_t bufs[4][128];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t q = blockIdx.x * 4 + warp, k = a.k;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *a.s.pool_next = 0;  // for the next stage
     if (q >= a.s.nq || *a.s.err) return;
+    if (a.ovf && a.ovf[q]) return;  // (nothing was recorded either: its bound is below every distance)
     uint64_t *buf = bufs[warp];
     CgList cg{};
     ExList ex{};
@@ -656,10 +686,14 @@ __global__ void __launch_bounds__(128) gt_replay_kernel(ReplayArgs a)
         const uint32_t c0 = uint32_t(li * T / a.s.W), c1 = uint32_t(((li + 1) * T - 1) / a.s.W);
         for (uint32_t s0 = c0; s0 <= c1; s0 += 32) {
             const uint32_t c = s0 + lane;
-            uint32_t cnt = c <= c1 ? a.s.list_n[size_t(c + li) * a.s.lrows + row] : 0u;
-            if (__any_sync(kFull, cnt > a.s.cap)) {
-                if (lane == 0) atomicExch(a.ovf, 1u);  // records lost: the host takes another engine
-                cnt = min(cnt, a.s.cap);
+            const uint32_t cnt = c <= c1 ? a.s.list_n[size_t(c + li) * a.s.lrows + row] : 0u;
+            if (__any_sync(kFull, cnt == SC_LOST)) {  // the host scans for this query again
+                if (lane == 0) {
+                    atomicExch(a.ovf ? a.any_ovf : a.s.err, 1u);
+                    if (a.ovf) a.ovf[q] = 1;
+                    a.bound[q] = -__int_as_float(0x7f800000);
+                }
+                return;
             }
             uint32_t incl = cnt;
 #pragma unroll
@@ -679,7 +713,12 @@ __global__ void __launch_bounds__(128) gt_replay_kernel(ReplayArgs a)
                 j = min(j, 31u);
                 const uint32_t off = e - __shfl_sync(kFull, excl, int(j));
                 uint2 rec = make_uint2(0u, 0u);
-                if (e < all) rec = a.s.lists[(size_t(s0 + j + li) * a.s.lrows + row) * a.s.cap + off];
+                if (e < all) {
+                    const size_t list = size_t(s0 + j + li) * a.s.lrows + row;
+                    const uint32_t x = off - a.s.cap;
+                    rec = off < a.s.cap ? a.s.lists[list * a.s.cap + off]
+                                        : a.s.pool[size_t(a.s.more[list * SC_MORE + x / SC_BLOCK]) * SC_BLOCK + x % SC_BLOCK];
+                }
                 if constexpr (EXACT) ex_batch(ex, buf, k, rec.x, rec.y, e < all, lane);
                 else cg_batch(cg, rec.x, rec.y, e < all, lane);
             }
@@ -689,6 +728,7 @@ __global__ void __launch_bounds__(128) gt_replay_kernel(ReplayArgs a)
         if (ex.fill) ex_flush(ex, buf, k, lane);
     if (a.last) {
         // output sorted by (dist, id) (CompGT.cpp:107-124)
+        const size_t out = size_t(a.rows ? a.rows[q] : q) * k;
         uint64_t key[4];
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
@@ -700,8 +740,8 @@ __global__ void __launch_bounds__(128) gt_replay_kernel(ReplayArgs a)
         for (int r = 0; r < 4; ++r) {
             const uint32_t i = r * 32 + lane;
             if (i < k) {
-                a.out_ids[size_t(q) * k + i] = key_id(key[r]);
-                a.out_dists[size_t(q) * k + i] = output_dist<MET>(key_dist(key[r]));
+                a.out_ids[out + i] = key_id(key[r]);
+                a.out_dists[out + i] = output_dist<MET>(key_dist(key[r]));
             }
         }
         return;
@@ -724,11 +764,11 @@ __global__ void __launch_bounds__(128) gt_replay_kernel(ReplayArgs a)
 // Codes -> bf16 rows of K elements (zero past the row), u8 centred by 128, and the row's value:
 // squared norm (L2); for u8 inner products the correction that undoes the centring, -128 * sum(b')
 // of a base row and -(128 * sum(q') + 128^2 * dims) of a query.  8 codes per thread: one 8-byte (4-bit:
-// 4-byte) load and one 16-byte store.
+// 4-byte) load and one 16-byte store.  pick: the source row of each row, or null.
 template <int DT>
 __global__ void __launch_bounds__(256) gt_codes_kernel(const uint8_t *src, uint32_t row_bytes, uint32_t stride, uint64_t rows,
                                                        uint64_t rows_pad, uint32_t K, uint32_t lr_log, uint32_t ip,
-                                                       uint32_t query, __nv_bfloat16 *dst, float *val)
+                                                       uint32_t query, const uint32_t *pick, __nv_bfloat16 *dst, float *val)
 {
     const uint64_t t = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     const uint32_t lr = 1u << lr_log;  // lanes per row: 8, 16 or 32
@@ -736,15 +776,16 @@ __global__ void __launch_bounds__(256) gt_codes_kernel(const uint8_t *src, uint3
     const uint32_t l = uint32_t(t) & (lr - 1);
     constexpr bool nib = DT == DT_U4;
     const uint32_t codes = nib ? row_bytes * 2 : row_bytes;
+    const uint8_t *const row = src + (pick && r < rows ? pick[r] : r) * stride;
     int32_t sq = 0, sum = 0;
     for (uint32_t g = l; g < K / 8; g += lr) {
         uint32_t w[2] = {0, 0};
         const bool in = r < rows && g * 8 < codes;  // whole groups lie within the padded row
         if (in) {
             if constexpr (nib) {
-                w[0] = *reinterpret_cast<const uint32_t *>(src + r * stride + g * 4);
+                w[0] = *reinterpret_cast<const uint32_t *>(row + g * 4);
             } else {
-                const uint2 x = *reinterpret_cast<const uint2 *>(src + r * stride + g * 8);
+                const uint2 x = *reinterpret_cast<const uint2 *>(row + g * 8);
                 w[0] = x.x;
                 w[1] = x.y;
             }
@@ -831,7 +872,7 @@ struct ScanSplit {
     uint32_t ctas, cap;
 };
 
-// One equal range of steps per SM; a range holds at most `most` records per query.
+// One equal range of steps per SM; the first block of a list holds `most` records, or all rows of a range.
 static ScanSplit scan_split(uint32_t qtiles, uint32_t T, uint32_t sms, uint32_t most)
 {
     ScanSplit s;
@@ -844,24 +885,14 @@ static ScanSplit scan_split(uint32_t qtiles, uint32_t T, uint32_t sms, uint32_t 
 
 size_t gt_tc_list_bytes(uint64_t n, uint32_t nq, uint32_t k, uint32_t sms);
 
-// Most records of one query in one range.  A stage records about 3 k rows of a query (15 k where k is small) over all
-// its ranges, two at least, so what the lists have past SC_CAP_MIN is room for rows in an order.  That room is given
-// within the memory that the replaying engine takes for its lists (up to 0.32, 0.64 or 1.27 GB for k up to 25, 51 and
-// above, on 152 SMs), less `other`, the rest of this scan's state.  Lists are kept for live queries only.
-static uint32_t scan_most(uint64_t n, uint32_t nq, uint32_t k, uint32_t sms, uint32_t batch, uint32_t lrows, size_t other)
-{
-    const size_t room = gt_tc_list_bytes(n, nq, k, sms);
-    const size_t per = size_t(sms + batch) * lrows * 8;
-    const size_t fit = room > other ? (room - other) / per / SC_ROWS * SC_ROWS : 0;
-    return uint32_t(std::min<size_t>(SC_CAP, std::max<size_t>(SC_CAP_MIN, fit)));
-}
-
 struct ScanLayout {
     uint32_t K, katoms, mt, qrows, batch;  // batch: query tiles per pass
-    uint32_t lrows, most;                  // queries of a tile that lists are kept for; their longest
+    uint32_t lrows;                        // queries of a tile that lists are kept for
     uint64_t n_pad, nq_pad;
     std::vector<uint32_t> at;
-    size_t off_q, off_bval, off_qval, off_flags, off_bound, off_d, off_i, off_top, off_dense, off_listn, off_lists, bytes;
+    size_t first, pool;  // records in the first blocks of all lists, and in the pool behind them
+    size_t off_q, off_bval, off_qval, off_flags, off_again, off_bound, off_d, off_i, off_top, off_dense, off_listn, off_more,
+        off_lists, bytes;
 };
 
 static ScanLayout scan_layout(uint32_t dtype, uint32_t dims, uint64_t n, uint32_t nq, uint32_t k, uint32_t sms)
@@ -878,28 +909,40 @@ static ScanLayout scan_layout(uint32_t dtype, uint32_t dims, uint64_t n, uint32_
     l.lrows = uint32_t(std::min<uint64_t>(nq, l.qrows));
     auto up = [](size_t x) { return (x + 255) / 256 * 256; };
     const size_t qb = std::min<size_t>(nq, size_t(l.batch) * l.qrows);
-    l.most = scan_most(n, nq, k, sms, l.batch, l.lrows, qb * (l.at[1] * SC_ROWS * 4 + 1036));
-    size_t lists = 0, segs = 0;
+    l.first = l.pool = 0;
     const uint64_t qtiles = l.nq_pad / l.qrows;
-    for (size_t i = 1; i + 1 < l.at.size(); ++i)
+    const size_t lists = l.at.size() > 2 ? size_t(sms + l.batch) * l.lrows : 0;
+    uint64_t rows = 0;  // of the longest stage
+    for (size_t i = 1; i + 1 < l.at.size(); ++i) {
+        rows = std::max(rows, uint64_t(l.at[i + 1] - l.at[i]) * SC_ROWS);
         for (uint64_t qt : {uint64_t(l.batch), qtiles % l.batch})  // a full batch and the last one
             if (qt) {
-                const ScanSplit s = scan_split(uint32_t(qt), l.at[i + 1] - l.at[i], sms, l.most);
-                lists = std::max(lists, size_t(s.ctas + qt) * l.lrows * s.cap);
-                segs = std::max(segs, size_t(s.ctas + qt) * l.lrows);
+                const ScanSplit s = scan_split(uint32_t(qt), l.at[i + 1] - l.at[i], sms, SC_FIRST);
+                l.first = std::max(l.first, size_t(s.ctas + qt) * l.lrows * s.cap);
             }
+    }
+    // A stage records about 3 k rows of a query (15 k where k is small) over all its ranges, two at least, so most
+    // lists end in their first block; the pool is for rows in an order.  It gets what is left of the memory that the
+    // replaying engine takes for its lists (up to 0.32, 0.64 or 1.27 GB for k up to 25, 51 and above, on 152 SMs), or
+    // 384 records per query where that is nothing, and never more than all rows of a stage.
+    const size_t room = gt_tc_list_bytes(n, nq, k, sms) / 8;
+    const size_t other = l.first + qb * (l.at[1] * SC_ROWS * 4 + 1036) / 8 + lists * (1 + SC_MORE) / 2;
+    l.pool = std::min<size_t>(qb * rows, std::max(qb * 384, room > other ? room - other : 0));
+    l.pool = (l.pool + SC_BLOCK - 1) / SC_BLOCK * SC_BLOCK;
     l.off_q = up(l.n_pad * l.K * 2);
     l.off_bval = l.off_q + up(l.nq_pad * l.K * 2);
     l.off_qval = l.off_bval + up(l.n_pad * 4);
     l.off_flags = l.off_qval + up(l.nq_pad * 4);
-    l.off_bound = l.off_flags + 256;
+    l.off_again = l.off_flags + up((4 + size_t(nq)) * 4);
+    l.off_bound = l.off_again + up(size_t(nq) * 4);
     l.off_d = l.off_bound + up(qb * 4);
     l.off_i = l.off_d + up(qb * 512);
     l.off_top = l.off_i + up(qb * 512);
     l.off_dense = l.off_top + up(qb * 8);
     l.off_listn = l.off_dense + up(qb * l.at[1] * SC_ROWS * 4);
-    l.off_lists = l.off_listn + up(segs * 4);
-    l.bytes = l.off_lists + up(lists * 8);
+    l.off_more = l.off_listn + up(lists * 4);
+    l.off_lists = l.off_more + up(lists * SC_MORE * 4);
+    l.bytes = l.off_lists + up((l.first + l.pool) * 8);
     return l;
 }
 
@@ -920,11 +963,28 @@ size_t gt_scan_workspace(uint32_t dtype, uint32_t dims, uint64_t n, uint32_t nq,
 
 template <int DT>
 static void launch_codes(const uint8_t *src, uint32_t dims, uint32_t stride, uint64_t rows, uint64_t rows_pad, uint32_t K,
-                         uint32_t ip, uint32_t query, __nv_bfloat16 *dst, float *val, cudaStream_t st)
+                         uint32_t ip, uint32_t query, const uint32_t *pick, __nv_bfloat16 *dst, float *val, cudaStream_t st)
 {
     const uint32_t lr_log = K == 64 ? 3 : K == 128 ? 4 : 5;
-    gt_codes_kernel<DT><<<uint32_t((rows_pad << lr_log) / 256), 256, 0, st>>>(src, dims, stride, rows, rows_pad, K, lr_log, ip, query,
+    gt_codes_kernel<DT><<<uint32_t((rows_pad << lr_log) / 256), 256, 0, st>>>(src, dims, stride, rows, rows_pad, K, lr_log, ip, query, pick,
                                                                       dst, val);
+}
+
+// Stages in which no first block can overflow, for `tiles` query tiles with lists for `lrows` queries of each: the
+// blocks of all ranges (one per SM at most) have room for every row of a range.
+static std::vector<uint32_t> scan_short_stages(const ScanLayout &l, uint32_t tiles, uint32_t lrows, uint32_t sms)
+{
+    const uint32_t T = l.at.back();
+    uint32_t len = T - l.at[1];
+    while (len > 1) {
+        const ScanSplit s = scan_split(tiles, len, sms, ~0u);
+        if (size_t(std::min<uint64_t>(sms, s.total) + tiles) * lrows * s.cap <= l.first + l.pool) break;
+        len = len * 7 / 8;
+    }
+    std::vector<uint32_t> at{0};
+    for (uint32_t b = l.at[1]; b < T; b += std::min(len, T - b)) at.push_back(b);
+    at.push_back(T);
+    return at;
 }
 
 template <bool EXACT>
@@ -937,16 +997,22 @@ static void launch_replay(uint32_t metric, const ReplayArgs &r, cudaStream_t st)
 
 // Device-resident inputs (rows of dims bytes, stride bytes apart); outputs device arrays nq * k.
 // ws: gt_scan_workspace() bytes, or NULL to allocate them here.  Returns after the work has finished
-// on `st`.  *overflow is set when a record list was too short (rows that come closer and closer to
-// a query, more of them in one range than a list holds): the outputs are then incomplete and the caller
-// takes an engine without lists.
+// on `st`.
+//
+// Rows in an order (a base stored by cluster, label or time) can come closer and closer to a query, more of them in
+// one range than there are blocks for.  Such queries record nothing in the stages that follow; at the end they are put
+// beside each other and scanned again, in stages so short that the first block of a list holds every row of a range.
+// *redone receives how many queries that were.  most_blocks: no more further blocks than that (for tests).
+// 10k x 1M x 128 u8 rows stored by label, k = 100 / 10: 16.5 / 19.7 ms (1,000 labels), 54 / 27 ms (64 labels, where
+// most queries fill the pool); in random order 4.2 / 3.0.  With lists of 4,096 and the replaying engine for every
+// query of the call behind them: 17.6 / 45 and 122 / 83.
 nbpg_status gt_scan_device(uint32_t dtype, uint32_t metric, uint32_t dims, uint32_t stride, const uint8_t *d_base,
                            uint64_t n, const uint8_t *d_q, uint32_t nq, uint32_t k, uint32_t mode, uint32_t *d_ids,
-                           float *d_dists, void *ws, cudaStream_t st, bool *overflow, bool withhold)
+                           float *d_dists, void *ws, cudaStream_t st, uint32_t *redone, uint32_t most_blocks, bool withhold)
 {
     const uint32_t sms = scan_sms();
     const ScanLayout l = scan_layout(dtype, dims, n, nq, k, sms);
-    *overflow = false;
+    if (redone) *redone = 0;
     auto fail = [](cudaError_t e) {
         set_error(std::string("nbpg_gt (tensor path): ") + cudaGetErrorString(e));
         return e == cudaErrorMemoryAllocation ? NBPG_ERR_OOM : NBPG_ERR_CUDA;
@@ -964,18 +1030,19 @@ nbpg_status gt_scan_device(uint32_t dtype, uint32_t metric, uint32_t dims, uint3
     uint8_t *w = static_cast<uint8_t *>(ws);
     __nv_bfloat16 *bB = reinterpret_cast<__nv_bfloat16 *>(w), *bQ = reinterpret_cast<__nv_bfloat16 *>(w + l.off_q);
     float *bval = reinterpret_cast<float *>(w + l.off_bval), *qval = reinterpret_cast<float *>(w + l.off_qval);
-    uint32_t *flags = reinterpret_cast<uint32_t *>(w + l.off_flags);  // [0] error, [1] overflow
+    uint32_t *flags = reinterpret_cast<uint32_t *>(w + l.off_flags);  // [0] error, [1] any overflow, [2] pool_next; from [4] per query
     nbpg_status s = NBPG_OK;
-    e = cudaMemsetAsync(flags, 0, 8, st);
+    e = cudaMemsetAsync(flags, 0, (4 + size_t(nq)) * 4, st);
     const uint32_t ip = metric == NBPG_IP;
+    auto codes = [&](const uint8_t *src, uint64_t rows, uint64_t pad, uint32_t query, const uint32_t *pick, __nv_bfloat16 *dst,
+                     float *val) {
+        if (dtype == NBPG_U8) launch_codes<DT_U8>(src, dims, stride, rows, pad, l.K, ip, query, pick, dst, val, st);
+        else if (dtype == NBPG_I8) launch_codes<DT_I8>(src, dims, stride, rows, pad, l.K, ip, query, pick, dst, val, st);
+        else launch_codes<DT_U4>(src, dims, stride, rows, pad, l.K, ip, query, pick, dst, val, st);
+    };
     if (e == cudaSuccess) {
-        auto codes = [&](const uint8_t *src, uint64_t rows, uint64_t pad, uint32_t query, __nv_bfloat16 *dst, float *val) {
-            if (dtype == NBPG_U8) launch_codes<DT_U8>(src, dims, stride, rows, pad, l.K, ip, query, dst, val, st);
-            else if (dtype == NBPG_I8) launch_codes<DT_I8>(src, dims, stride, rows, pad, l.K, ip, query, dst, val, st);
-            else launch_codes<DT_U4>(src, dims, stride, rows, pad, l.K, ip, query, dst, val, st);
-        };
-        codes(d_base, n, l.n_pad, 0, bB, bval);
-        codes(d_q, nq, l.nq_pad, 1, bQ, qval);
+        codes(d_base, n, l.n_pad, 0, nullptr, bB, bval);
+        codes(d_q, nq, l.nq_pad, 1, nullptr, bQ, qval);
         e = cudaGetLastError();
     }
     CUtensorMap mA, mB;
@@ -1015,48 +1082,76 @@ nbpg_status gt_scan_device(uint32_t dtype, uint32_t metric, uint32_t dims, uint3
     r.s.list_n = reinterpret_cast<uint32_t *>(w + l.off_listn);
     r.s.dense = reinterpret_cast<float *>(w + l.off_dense);
     r.s.dense_stride = l.at[1] * SC_ROWS;
-    r.s.lrows = l.lrows;
+    r.s.more = reinterpret_cast<uint32_t *>(w + l.off_more);
+    r.s.pool = r.s.lists + l.first;
+    r.s.pool_next = flags + 2;
     r.s.err = flags;
     r.k = k;
     r.st_d = reinterpret_cast<uint4 *>(w + l.off_d);
     r.st_i = reinterpret_cast<uint4 *>(w + l.off_i);
     r.st_top = reinterpret_cast<uint2 *>(w + l.off_top);
-    r.ovf = flags + 1;
-    const uint64_t per_batch = uint64_t(l.batch) * l.qrows;
-    for (uint64_t q0 = 0; e == cudaSuccess && s == NBPG_OK && q0 < nq; q0 += per_batch) {
-        r.s.nq = uint32_t(std::min<uint64_t>(per_batch, nq - q0));
-        r.s.qval = qval + q0;
-        r.s.q_row0 = uint32_t(q0);
-        r.out_ids = d_ids + q0 * k;
-        r.out_dists = d_dists + q0 * k;
-        const uint32_t qtiles = (r.s.nq + l.qrows - 1) / l.qrows;
-        for (size_t i = 0; i + 1 < l.at.size(); ++i) {
-            r.s.b_first = l.at[i];
-            r.s.T = l.at[i + 1] - l.at[i];
-            const ScanSplit sp = scan_split(qtiles, r.s.T, sms, l.most);
-            r.s.W = sp.W;
-            r.s.total = sp.total;
-            r.s.cap = sp.cap;
-            r.first = i == 0;
-            r.last = i + 2 == l.at.size();
-            if (r.first) gt_scan_kernel<true><<<sp.ctas, SC_THREADS, smem, st>>>(mA, mB, r.s);
-            else gt_scan_kernel<false><<<sp.ctas, SC_THREADS, smem, st>>>(mA, mB, r.s);
-            if (mode == NBPG_GT_EXACT) launch_replay<true>(metric, r, st);
-            else launch_replay<false>(metric, r, st);
+    r.any_ovf = flags + 1;
+    // all stages for the first `count` converted queries; outputs in the rows `rows`, or as they come
+    auto pass = [&](uint32_t count, const uint32_t *rows) {
+        const uint64_t per_batch = uint64_t(l.batch) * l.qrows;
+        for (uint64_t q0 = 0; e == cudaSuccess && q0 < count; q0 += per_batch) {
+            r.s.nq = uint32_t(std::min<uint64_t>(per_batch, count - q0));
+            r.s.qval = qval + q0;
+            r.s.q_row0 = uint32_t(q0);
+            r.rows = rows ? rows + q0 : nullptr;
+            r.ovf = rows ? nullptr : flags + 4 + q0;
+            r.out_ids = d_ids + (rows ? 0 : q0 * k);
+            r.out_dists = d_dists + (rows ? 0 : q0 * k);
+            const uint32_t qtiles = (r.s.nq + l.qrows - 1) / l.qrows;
+            r.s.lrows = std::min(count, l.qrows);
+            r.s.pool_blocks = rows ? 0u : uint32_t(std::min<size_t>(l.pool / SC_BLOCK, most_blocks));
+            const std::vector<uint32_t> at = rows ? scan_short_stages(l, qtiles, r.s.lrows, sms) : l.at;
+            for (size_t i = 0; i + 1 < at.size(); ++i) {
+                r.s.b_first = at[i];
+                r.s.T = at[i + 1] - at[i];
+                const ScanSplit sp = scan_split(qtiles, r.s.T, sms, rows ? ~0u : SC_FIRST);
+                r.s.W = sp.W;
+                r.s.total = sp.total;
+                r.s.cap = sp.cap;
+                r.first = i == 0;
+                r.last = i + 2 == at.size();
+                if (r.first) gt_scan_kernel<true><<<sp.ctas, SC_THREADS, smem, st>>>(mA, mB, r.s);
+                else gt_scan_kernel<false><<<sp.ctas, SC_THREADS, smem, st>>>(mA, mB, r.s);
+                if (mode == NBPG_GT_EXACT) launch_replay<true>(metric, r, st);
+                else launch_replay<false>(metric, r, st);
+            }
+            e = cudaGetLastError();
         }
-        e = cudaGetLastError();
-    }
+    };
     uint32_t h[2] = {0, 0};
-    if (e == cudaSuccess && s == NBPG_OK) e = cudaMemcpyAsync(h, flags, 8, cudaMemcpyDeviceToHost, st);
-    const cudaError_t es = cudaStreamSynchronize(st);
-    if (e == cudaSuccess) e = es;
+    auto finish = [&](void *to, const void *from, size_t bytes) {
+        if (e == cudaSuccess && s == NBPG_OK) e = cudaMemcpyAsync(to, from, bytes, cudaMemcpyDeviceToHost, st);
+        const cudaError_t es = cudaStreamSynchronize(st);
+        if (e == cudaSuccess) e = es;
+    };
+    if (s == NBPG_OK) pass(nq, nullptr);
+    finish(h, flags, 8);
+    if (e == cudaSuccess && s == NBPG_OK && !h[0] && h[1]) {
+        std::vector<uint32_t> ovf(nq), rows;
+        finish(ovf.data(), flags + 4, size_t(nq) * 4);
+        for (uint32_t q = 0; q < nq; ++q)
+            if (ovf[q]) rows.push_back(q);
+        if (redone) *redone = uint32_t(rows.size());
+        uint32_t *d_rows = reinterpret_cast<uint32_t *>(w + l.off_again);
+        const uint32_t m = uint32_t(rows.size());
+        if (e == cudaSuccess) e = cudaMemcpyAsync(d_rows, rows.data(), size_t(m) * 4, cudaMemcpyHostToDevice, st);
+        if (e == cudaSuccess) {
+            codes(d_q, m, (uint64_t(m) + l.qrows - 1) / l.qrows * l.qrows, 1, d_rows, bQ, qval);
+            pass(m, d_rows);
+        }
+        finish(h, flags, 8);
+    }
     if (owned) cudaFree(owned);
     if (e != cudaSuccess && s == NBPG_OK) s = fail(e);
     if (s == NBPG_OK && h[0]) {
         set_error("nbpg_gt (tensor path): a pipeline wait timed out");
         s = NBPG_ERR_TIMEOUT;
     }
-    *overflow = h[1] != 0;
     return s;
 }
 
@@ -1081,10 +1176,9 @@ extern "C" nbpg_status nbpg_test_gt_timeout(int32_t device)
     if (e == cudaSuccess) e = cudaMemset(db, 7, n * dims);
     if (e == cudaSuccess) e = cudaMemset(dq, 3, nq * dims);
     nbpg_status s = NBPG_ERR_CUDA;
-    bool overflow = false;
     if (e == cudaSuccess)
         s = gt_scan_device(NBPG_U8, NBPG_L2, dims, dims, db, n, dq, nq, k, NBPG_GT_COMPGT, di, dd, nullptr, nullptr,
-                           &overflow, true);
+                           nullptr, ~0u, true);
     cudaFree(db);
     cudaFree(dq);
     cudaFree(di);

@@ -1,10 +1,9 @@
 // Brute-force kNN with tcgen05 tensor cores, replaying as it scans: compute_groundtruth
 // (data_tools/ANNs/data_proc/CompGT.cpp:29-134), same outputs as gt.cu.
 //
-// Runs when a record list of the staged scan (gt_scan.cu) overflows: rows ordered so that thousands
-// in one range come closer and closer to a query.  Here most of those are admitted where they are
-// met, without a list.  On rows in random order the staged scan is the faster one (10k x 1M x 128,
-// k = 100: 4.2 ms against 9.6).
+// Runs where the memory of the staged scan (gt_scan.cu) is not to be had and this engine's is: some
+// sizes below 1M rows take up to 75 MB less here.  Otherwise the staged scan is the faster one (10k x
+// 1M x 128, k = 100: 4.2 ms against 9.6).
 //
 // Exactness: u8 (0..255), i8 (-128..127) and 4-bit codes are exact in bf16, their
 // products are exact in fp32, and every partial sum of a row's dot product stays an
