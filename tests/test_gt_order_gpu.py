@@ -65,3 +65,29 @@ def test_gt_some_queries_again(gpu_lib, nq, step):
     for exact in (False, True):
         redone = _redone(gpu_lib, b, q, "u8", "l2", 10, exact, (ALL, 0))
         assert redone[1] == len(near), redone
+
+
+@pytest.mark.parametrize("n,dims,nq,k", [(1171, 256, 1, 100), (1172, 256, 1, 100), (390, 256, 2, 16), (391, 256, 2, 16),
+                                         (390, 256, 2, 17), (129, 130, 1, 128), (300, 576, 40, 10)])
+def test_gt_small_calls_with_and_without_a_workspace(gpu_lib, n, dims, nq, k):
+    """The sizes around which a call without a workspace goes to DP4A instead of allocating one"""
+    import torch
+    from nbpg_gb300.index import ground_truth_device, gt_workspace_size
+    stride = (dims + 15) // 16 * 16
+    g = torch.Generator(device="cuda").manual_seed(n)
+    x = torch.randint(0, 256, (n + nq, stride), generator=g, device="cuda", dtype=torch.uint8)
+    x[:, dims:] = 0
+    ws = torch.empty(gt_workspace_size("u8", dims, n, nq, k), dtype=torch.uint8, device="cuda")
+    assert ws.numel() > 0
+    torch.cuda.synchronize()
+    for exact in (False, True):
+        out = []
+        for w, engine in ((ws, "auto"), (None, "auto"), (None, "dp4a")):
+            ids = torch.empty((nq, k), dtype=torch.int32, device="cuda")
+            ds = torch.empty((nq, k), dtype=torch.float32, device="cuda")
+            ground_truth_device(x.data_ptr(), n, x[n:].data_ptr(), nq, dims, stride, "u8", "l2", k, ids.data_ptr(),
+                                ds.data_ptr(), exact=exact, engine=engine, d_workspace=w.data_ptr() if w is not None else 0,
+                                workspace_bytes=ws.numel() if w is not None else 0)
+            out.append((ids, ds))
+        for ids, ds in out[1:]:
+            assert torch.equal(ids, out[0][0]) and torch.equal(ds, out[0][1]), exact
