@@ -402,7 +402,7 @@ static nbpg_status build_impl(nbpg_index *idx, const nbpg_build_params &P, nbpg_
     bool flag = VL >= L && P.dir_bias_scale <= 0;
     SlotLayout flay{};
     PruneLayout play{};
-    uint32_t fw = 0, fgrid = 0;  // warps per CTA, CTAs
+    uint32_t fw = 0, fgrid = 0, fout = 0;  // warps per CTA, CTAs, warps per CTA with a filter in global memory
     size_t fsmem = 0;
     BuildFlagArgs F{};
     F.B.s = sa;
@@ -418,22 +418,14 @@ static nbpg_status build_impl(nbpg_index *idx, const nbpg_build_params &P, nbpg_
         F.lay_g = make_flag_layout(L, R, idx->row_stride, false, S, false);
         F.own = ghash ? 0 : std::min<uint32_t>(16, uint32_t(idx->smem_optin / flay.bytes));
         const size_t left = idx->smem_optin - F.own * size_t(flay.bytes);
-        const uint32_t out = std::min<uint32_t>(16 - F.own, uint32_t(left / F.lay_g.bytes));
-        fw = F.own + out;
-        fsmem = F.own * size_t(flay.bytes) + out * size_t(F.lay_g.bytes);
+        fout = std::min<uint32_t>(16 - F.own, uint32_t(left / F.lay_g.bytes));
+        fw = F.own + fout;
+        fsmem = F.own * size_t(flay.bytes) + fout * size_t(F.lay_g.bytes);
         int fb = 0;
         NBPG_CUDA_TRY(build_flag_search(idx->desc.dtype, idx->desc.metric, 0, fw, fsmem, F, &fb, st));
         NBPG_CUDA_TRY(build_flag_prune(idx->desc.dtype, idx->desc.metric, 0, F, play, st));
         flag = fb >= 1;
         fgrid = uint32_t(fb) * uint32_t(idx->sm_count);
-        if (flag && out) {
-            if (idx->ghash.ensure(std::max(ghash ? nslots : 0, size_t(fgrid) * out) * S * 4) != NBPG_OK) {
-                cudaGetLastError();  // no room: the one-kernel insert needs less
-                flag = false;
-                if (ghash && (s = idx->ghash.ensure(nslots * S * 4)) != NBPG_OK) return s;
-            }
-            if (ghash) sa.g_hash = idx->ghash.as<uint32_t>();
-        }
     }
 
     // batch size (nsw.h:288-295): min(0.02 * n (through float), 1e6), at least 1
@@ -453,6 +445,20 @@ static nbpg_status build_impl(nbpg_index *idx, const nbpg_build_params &P, nbpg_
         (s = d_off.ensure(n * 4)) || (s = d_bump.ensure(32)) || (s = d_grp.ensure(eff * R * 4)) ||
         (s = d_edges.ensure(eff * R * 8)))
         return fail_oom(s);
+    // FGIM: the graph the pair passes write (toG), which becomes the index's graph
+    DevBuf d_tog;
+    ReleaseOnExit release_tog{{&d_tog}};
+    if (fgim && (s = d_tog.ensure(size_t(n) * idx->gstride * 4)) != NBPG_OK) return s;
+    if (P.dir_bias_scale > 0 && (s = d_bias.ensure(size_t(R + 1) * sizeof(double))) != NBPG_OK) return s;
+    // What follows makes the build faster and is left out where it does not fit, so it comes after all that is needed.
+    if (flag && fout) {
+        if (idx->ghash.ensure(std::max(ghash ? nslots : 0, size_t(fgrid) * fout) * S * 4) != NBPG_OK) {
+            cudaGetLastError();  // no room: the one-kernel insert needs less
+            flag = false;
+            if (ghash && (s = idx->ghash.ensure(nslots * S * 4)) != NBPG_OK) return s;
+        }
+        if (ghash) sa.g_hash = idx->ghash.as<uint32_t>();
+    }
     NBPG_CUDA_TRY(cudaMemsetAsync(d_cnt.ptr, 0, n * 4, st));
     NBPG_CUDA_TRY(cudaMemsetAsync(d_sv.ptr, 0, n * 4, st));
     NBPG_CUDA_TRY(cudaMemsetAsync(d_sd.ptr, 0, n * 4, st));
@@ -505,7 +511,6 @@ static nbpg_status build_impl(nbpg_index *idx, const nbpg_build_params &P, nbpg_
         // widened as the reference's expression widens it (prune.h:59-63); a degree is at most R
         bias_host.resize(R + 1);
         for (uint32_t d = 0; d <= R; ++d) bias_host[d] = P.dir_bias_scale * std::log(double(d + 1)) + 1;
-        if ((s = d_bias.ensure(size_t(R + 1) * sizeof(double))) != NBPG_OK) return s;
         NBPG_CUDA_TRY(cudaMemcpyAsync(d_bias.ptr, bias_host.data(), size_t(R + 1) * sizeof(double),
                                       cudaMemcpyHostToDevice, st));
         B.dir_bias = d_bias.as<double>();
@@ -521,12 +526,8 @@ static nbpg_status build_impl(nbpg_index *idx, const nbpg_build_params &P, nbpg_
     std::mt19937 sp_engine{uint32_t(P.sp_seed)};
     uint64_t batches = 0;
 
-    // FGIM: the graph the pair passes write (toG), which becomes the index's graph
-    DevBuf d_tog;
-    ReleaseOnExit release_tog{{&d_tog}};
     uint32_t *tog = nullptr;
     if (fgim) {
-        if ((s = d_tog.ensure(size_t(n) * idx->gstride * 4)) != NBPG_OK) return s;
         tog = d_tog.as<uint32_t>();
         NBPG_CUDA_TRY(cudaMemsetAsync(tog, 0, size_t(n) * idx->gstride * 4, st));
     }

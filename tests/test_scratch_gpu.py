@@ -97,3 +97,34 @@ shim.shim_limit(1 << 40)
 got = ground_truth(base, base[:1], "u8", "l2", k=100)
 assert np.array_equal(got[0], want[0]) and shim.shim_overrun() == 0 and shim.shim_peak() > 0
 """)
+
+
+@pytest.mark.parametrize("fgim", [False, True])
+def test_build_leaves_out_what_does_not_fit(shim, fgim):
+    """The neighbours' distances (n x R x 4 bytes) and the insert's key buffers only make the build faster: with less
+    memory than they take the build runs without them and gives the same graph, until what it needs does not fit."""
+    shim(f"fgim = {fgim}" + """
+n, R = 20000, 32
+base, _ = synth.u8_mixture(n, 1, dim=32, n_centres=32)
+def build(limit):
+    idx = Index(base, "u8", "l2", max_degree=R)
+    shim.shim_limit(limit)
+    shim.shim_reset_peak()
+    try:
+        (idx.build_fgim if fgim else idx.build_vamana)(L=40, VL=60, num_split=2 if fgim else 0, num_passes=2)
+        g = idx.get_graph()
+        return shim.shim_peak(), [tuple(r[1:1 + r[0]]) for r in g]
+    except _lib.NbpgError as e:
+        assert e.status == 2
+        return None
+    finally:
+        shim.shim_limit(1 << 40)
+        idx.close()
+peak, want = build(1 << 40)
+room = n * R * 4
+for limit in (peak - 1, peak - room // 2, peak - room):
+    used, got = build(limit)
+    assert used <= limit and got == want
+assert build(peak // 3) is None
+assert build(1 << 40)[1] == want and shim.shim_overrun() == 0
+""")
