@@ -176,45 +176,70 @@ static __global__ void rows_scatter_kernel(uint32_t *graph, uint32_t gstride, ui
         graph[size_t(ids[blockIdx.x]) * gstride + j] = in[size_t(blockIdx.x) * words + j];
 }
 
-// Host copies of graph rows, fetched when first asked for and written back together
-struct RowCache {
+// Host copies of graph rows: of those asked for, through the device's gather and scatter, or of the whole graph
+struct HostRows {
     nbpg_index *idx;
+    bool whole = false;
     std::unordered_map<uint32_t, uint32_t> at;  // node -> row in `rows`
     std::vector<uint32_t> ids, rows;
     DevBuf d_ids, d_rows;
     ReleaseOnExit release{{&d_ids, &d_rows}};
+    explicit HostRows(nbpg_index *i) : idx(i) {}
     uint32_t words() const { return idx->desc.max_degree + 1; }
-    nbpg_status fetch(const std::vector<uint32_t> &want)
+    bool has(uint32_t v) const { return whole || at.find(v) != at.end(); }
+    uint32_t *row(uint32_t v) { return &rows[size_t(whole ? v : at.at(v)) * words()]; }
+
+    nbpg_status fetch_all()
     {
-        std::vector<uint32_t> miss;
-        for (uint32_t v : want)
-            if (at.emplace(v, uint32_t(ids.size() + miss.size())).second) miss.push_back(v);
-        if (miss.empty()) return NBPG_OK;
-        nbpg_status s;
-        const size_t bytes = miss.size() * words() * 4;
-        if ((s = d_ids.ensure(miss.size() * 4)) || (s = d_rows.ensure(bytes))) return s;
-        NBPG_CUDA_TRY(cudaMemcpyAsync(d_ids.ptr, miss.data(), miss.size() * 4, cudaMemcpyHostToDevice, idx->stream));
-        rows_gather_kernel<<<uint32_t(miss.size()), 64, 0, idx->stream>>>(idx->d_graph, idx->gstride, words(),
-                                                                          d_ids.as<uint32_t>(), d_rows.as<uint32_t>());
-        NBPG_CUDA_TRY(cudaGetLastError());
-        const size_t old = rows.size();
-        rows.resize(old + miss.size() * words());
-        NBPG_CUDA_TRY(cudaMemcpyAsync(rows.data() + old, d_rows.ptr, bytes, cudaMemcpyDeviceToHost, idx->stream));
+        rows.resize(size_t(idx->desc.n) * words());
+        NBPG_CUDA_TRY(cudaMemcpy2DAsync(rows.data(), words() * 4, idx->d_graph, idx->gstride * 4, words() * 4, idx->desc.n,
+                                        cudaMemcpyDeviceToHost, idx->stream));
         NBPG_CUDA_TRY(cudaStreamSynchronize(idx->stream));
-        ids.insert(ids.end(), miss.begin(), miss.end());
+        whole = true;
         return NBPG_OK;
     }
-    uint32_t *row(uint32_t v) { return &rows[size_t(at.at(v)) * words()]; }
+    // between the rows ids[first, ids.size()) and the device, a piece at a time: pieces shrink to the room there is
+    nbpg_status move(size_t first, bool back)
+    {
+        size_t piece = std::min<size_t>(ids.size() - first, 65536);
+        while (d_ids.ensure(piece * 4) != NBPG_OK || d_rows.ensure(piece * words() * 4) != NBPG_OK) {
+            cudaGetLastError();
+            if (piece <= 64) return NBPG_ERR_OOM;
+            piece /= 2;
+        }
+        cudaStream_t st = idx->stream;
+        for (size_t i = first; i < ids.size(); i += piece) {
+            const uint32_t cnt = uint32_t(std::min(piece, ids.size() - i));
+            uint32_t *host = rows.data() + i * words();
+            const size_t bytes = size_t(cnt) * words() * 4;
+            NBPG_CUDA_TRY(cudaMemcpyAsync(d_ids.ptr, ids.data() + i, size_t(cnt) * 4, cudaMemcpyHostToDevice, st));
+            if (back) NBPG_CUDA_TRY(cudaMemcpyAsync(d_rows.ptr, host, bytes, cudaMemcpyHostToDevice, st));
+            if (back)
+                rows_scatter_kernel<<<cnt, 64, 0, st>>>(idx->d_graph, idx->gstride, words(), d_ids.as<uint32_t>(),
+                                                        d_rows.as<uint32_t>());
+            else
+                rows_gather_kernel<<<cnt, 64, 0, st>>>(idx->d_graph, idx->gstride, words(), d_ids.as<uint32_t>(),
+                                                       d_rows.as<uint32_t>());
+            NBPG_CUDA_TRY(cudaGetLastError());
+            if (!back) NBPG_CUDA_TRY(cudaMemcpyAsync(host, d_rows.ptr, bytes, cudaMemcpyDeviceToHost, st));
+            NBPG_CUDA_TRY(cudaStreamSynchronize(st));
+        }
+        return NBPG_OK;
+    }
+    nbpg_status fetch(const std::vector<uint32_t> &want)
+    {
+        if (whole) return NBPG_OK;
+        const size_t old = ids.size();
+        for (uint32_t v : want)
+            if (at.emplace(v, uint32_t(ids.size())).second) ids.push_back(v);
+        rows.resize(ids.size() * words());
+        return old < ids.size() ? move(old, false) : NBPG_OK;
+    }
     nbpg_status write_back()
     {
-        if (ids.empty()) return NBPG_OK;
-        nbpg_status s;
-        if ((s = d_ids.ensure(ids.size() * 4)) || (s = d_rows.ensure(rows.size() * 4))) return s;
-        NBPG_CUDA_TRY(cudaMemcpyAsync(d_ids.ptr, ids.data(), ids.size() * 4, cudaMemcpyHostToDevice, idx->stream));
-        NBPG_CUDA_TRY(cudaMemcpyAsync(d_rows.ptr, rows.data(), rows.size() * 4, cudaMemcpyHostToDevice, idx->stream));
-        rows_scatter_kernel<<<uint32_t(ids.size()), 64, 0, idx->stream>>>(idx->d_graph, idx->gstride, words(),
-                                                                          d_ids.as<uint32_t>(), d_rows.as<uint32_t>());
-        NBPG_CUDA_TRY(cudaGetLastError());
+        if (!whole) return move(0, true);
+        NBPG_CUDA_TRY(cudaMemcpy2DAsync(idx->d_graph, idx->gstride * 4, rows.data(), words() * 4, words() * 4, idx->desc.n,
+                                        cudaMemcpyHostToDevice, idx->stream));
         NBPG_CUDA_TRY(cudaStreamSynchronize(idx->stream));
         return NBPG_OK;
     }
@@ -231,24 +256,26 @@ static bool add_edge_if_possible(uint32_t *r, uint32_t R, uint32_t to)
     return true;
 }
 
-// Every node unreachable from the entry gets an in-edge; *count receives how many there were.
-static nbpg_status repair_isolated(nbpg_index *idx, uint32_t entry, uint64_t *count)
+// The nodes reachable from the entry, as bits; *swept is false where the device's sweep is too deep or has no room
+static nbpg_status reach_sweep(nbpg_index *idx, uint32_t entry, std::vector<uint32_t> &seen, bool *swept)
 {
-    const uint32_t R = idx->desc.max_degree, n = uint32_t(idx->desc.n);
-    const size_t words = (size_t(n) + 31) / 32;
+    const uint32_t n = uint32_t(idx->desc.n);
     cudaStream_t st = idx->stream;
     DevBuf d_seen, d_queue, d_head;
     ReleaseOnExit release{{&d_seen, &d_queue, &d_head}};
-    nbpg_status s;
     const size_t heads = REACH_MOST + 2;
-    if ((s = d_seen.ensure(words * 4)) || (s = d_queue.ensure(size_t(n) * 4)) || (s = d_head.ensure(heads * 4))) return s;
-    NBPG_CUDA_TRY(cudaMemsetAsync(d_seen.ptr, 0, words * 4, st));
+    *swept = false;
+    if (d_seen.ensure(seen.size() * 4) != NBPG_OK || d_queue.ensure(size_t(n) * 4) != NBPG_OK ||
+        d_head.ensure(heads * 4) != NBPG_OK) {
+        cudaGetLastError();
+        return NBPG_OK;
+    }
+    NBPG_CUDA_TRY(cudaMemsetAsync(d_seen.ptr, 0, seen.size() * 4, st));
     NBPG_CUDA_TRY(cudaMemsetAsync(d_head.ptr, 0, heads * 4, st));
     uint32_t *head = d_head.as<uint32_t>();
     reach_start_kernel<<<1, 1, 0, st>>>(d_seen.as<uint32_t>(), d_queue.as<uint32_t>(), head, entry);
     const uint32_t grid = uint32_t(std::min<size_t>(size_t(idx->sm_count) * 8, size_t(n) / 8 + 1));
-    bool swept = false;
-    for (uint32_t level = 0; level < REACH_MOST && !swept; ++level) {
+    for (uint32_t level = 0; level < REACH_MOST && !*swept; ++level) {
         reach_level_kernel<<<grid, 256, 0, st>>>(idx->d_graph, idx->gstride, d_seen.as<uint32_t>(), d_queue.as<uint32_t>(),
                                                  head, level);
         reach_close_kernel<<<1, 1, 0, st>>>(head, level);
@@ -257,77 +284,90 @@ static nbpg_status repair_isolated(nbpg_index *idx, uint32_t entry, uint64_t *co
             uint32_t h[2];
             NBPG_CUDA_TRY(cudaMemcpyAsync(h, head + level + 1, 8, cudaMemcpyDeviceToHost, st));
             NBPG_CUDA_TRY(cudaStreamSynchronize(st));
-            swept = h[0] == h[1];  // the last level found nothing new
+            *swept = h[0] == h[1];  // the last level found nothing new
         }
     }
-    std::vector<uint32_t> seen(words, 0u);
-    if (swept) {
-        NBPG_CUDA_TRY(cudaMemcpyAsync(seen.data(), d_seen.ptr, words * 4, cudaMemcpyDeviceToHost, st));
+    if (*swept) {
+        NBPG_CUDA_TRY(cudaMemcpyAsync(seen.data(), d_seen.ptr, seen.size() * 4, cudaMemcpyDeviceToHost, st));
         NBPG_CUDA_TRY(cudaStreamSynchronize(st));
-    } else {
-        std::vector<uint32_t> G(size_t(n) * (R + 1)), queue{entry};
-        NBPG_CUDA_TRY(cudaMemcpy2DAsync(G.data(), (R + 1) * 4, idx->d_graph, idx->gstride * 4, (R + 1) * 4, n,
-                                        cudaMemcpyDeviceToHost, st));
-        NBPG_CUDA_TRY(cudaStreamSynchronize(st));
+    }
+    return NBPG_OK;
+}
+
+// Every node unreachable from the entry gets an in-edge; *count receives how many there were.
+static nbpg_status repair_isolated(nbpg_index *idx, uint32_t entry, uint64_t *count)
+{
+    const uint32_t R = idx->desc.max_degree, n = uint32_t(idx->desc.n);
+    std::vector<uint32_t> seen((size_t(n) + 31) / 32, 0u);
+    auto reached = [&](uint32_t v) { return ((seen[v >> 5] >> (v & 31)) & 1) != 0; };
+    HostRows rows(idx);
+    bool swept = false;
+    nbpg_status s = reach_sweep(idx, entry, seen, &swept);
+    if (s != NBPG_OK) return s;
+    if (!swept) {
+        if ((s = rows.fetch_all()) != NBPG_OK) return s;
+        std::vector<uint32_t> queue{entry};
         seen[entry >> 5] |= 1u << (entry & 31);
         for (size_t h = 0; h < queue.size(); ++h) {
-            const uint32_t *r = &G[size_t(queue[h]) * (R + 1)];
-            for (uint32_t j = 0; j < r[0]; ++j) {
-                const uint32_t v = r[1 + j], bit = 1u << (v & 31);
-                if (!(seen[v >> 5] & bit)) {
-                    seen[v >> 5] |= bit;
-                    queue.push_back(v);
+            const uint32_t *r = rows.row(queue[h]);
+            for (uint32_t j = 0; j < r[0]; ++j)
+                if (!reached(r[1 + j])) {
+                    seen[r[1 + j] >> 5] |= 1u << (r[1 + j] & 31);
+                    queue.push_back(r[1 + j]);
                 }
-            }
         }
     }
-    auto reached = [&](uint32_t v) { return ((seen[v >> 5] >> (v & 31)) & 1) != 0; };
     std::vector<uint32_t> lost;
-    for (uint32_t w = 0; w < words; ++w) {
+    for (uint32_t w = 0; w < seen.size(); ++w) {
         uint32_t m = ~seen[w];
         if (size_t(w) * 32 + 32 > n) m &= (1u << (n & 31)) - 1u;
         for (; m; m &= m - 1) lost.push_back(w * 32 + uint32_t(__builtin_ctz(m)));
     }
     *count = lost.size();
     if (lost.empty()) return NBPG_OK;
-    // the rows the repair reads and writes: the lost nodes', their neighbours' and the entry's
-    RowCache rc{idx, {}, {}, {}, {}, {}};
-    std::vector<uint32_t> want(lost);
-    want.push_back(entry);
-    if ((s = rc.fetch(want)) != NBPG_OK) return s;
-    want.clear();
-    for (uint32_t i : lost) {
-        const uint32_t *r = rc.row(i);
-        want.insert(want.end(), r + 1, r + 1 + r[0]);
+    // The rows the repair reads and writes: the lost nodes', their neighbours' and the entry's.  From about a 128th of
+    // the graph on, one copy of it is cheaper than looking each row up (1M rows of R = 32, by rows / by the copy: one in
+    // 64 lost 78 / 48 ms, one in 1,000 6 / 48, all 2,071 / 236).
+    if (lost.size() > n / 128 && !rows.whole && (s = rows.fetch_all()) != NBPG_OK) return s;
+    if (!rows.whole) {
+        std::vector<uint32_t> want(lost);
+        want.push_back(entry);
+        if ((s = rows.fetch(want)) != NBPG_OK) return s;
+        want.clear();
+        for (uint32_t i : lost) {
+            const uint32_t *r = rows.row(i);
+            want.insert(want.end(), r + 1, r + 1 + r[0]);
+        }
+        if ((s = rows.fetch(want)) != NBPG_OK) return s;
     }
-    if ((s = rc.fetch(want)) != NBPG_OK) return s;
+    uint32_t open = 0;  // no reached node before it has room for an edge, and none gets any
     for (uint32_t i : lost) {
         // a neighbour list of its own: adding an edge below can lengthen this node's row while it is walked
         // only by the node itself, which add_edge_if_possible refuses to repeat
         bool done = false;
-        for (uint32_t j = 0; j < rc.row(i)[0] && !done; ++j) {
-            const uint32_t v = rc.row(i)[1 + j];
-            if (reached(v)) done = add_edge_if_possible(rc.row(v), R, i);
+        for (uint32_t j = 0; j < rows.row(i)[0] && !done; ++j) {
+            const uint32_t v = rows.row(i)[1 + j];
+            if (reached(v)) done = add_edge_if_possible(rows.row(v), R, i);
         }
-        for (uint32_t j = 0; j < rc.row(i)[0] && !done; ++j) {
-            const uint32_t v = rc.row(i)[1 + j];
-            if (rc.at.find(v) == rc.at.end() && (s = rc.fetch({v})) != NBPG_OK) return s;
-            done = add_edge_if_possible(rc.row(v), R, i);
+        for (uint32_t j = 0; j < rows.row(i)[0] && !done; ++j) {
+            const uint32_t v = rows.row(i)[1 + j];
+            if (!rows.has(v) && (s = rows.fetch({v})) != NBPG_OK) return s;
+            done = add_edge_if_possible(rows.row(v), R, i);
         }
-        if (!done) done = add_edge_if_possible(rc.row(entry), R, i);
-        for (uint32_t x = 0; x < n && !done; ++x) {
-            if (!reached(x)) continue;
-            if (rc.at.find(x) == rc.at.end()) {
+        if (!done) done = add_edge_if_possible(rows.row(entry), R, i);
+        for (; open < n && !done; ++open) {  // (a full row refuses every edge, so the place is kept between nodes)
+            if (!reached(open)) continue;
+            if (!rows.has(open)) {
                 // the nodes from here on, a thousand at a time
                 std::vector<uint32_t> next;
-                for (uint32_t y = x; y < n && next.size() < 1024; ++y)
+                for (uint32_t y = open; y < n && next.size() < 1024; ++y)
                     if (reached(y)) next.push_back(y);
-                if ((s = rc.fetch(next)) != NBPG_OK) return s;
+                if ((s = rows.fetch(next)) != NBPG_OK) return s;
             }
-            done = add_edge_if_possible(rc.row(x), R, i);
+            if ((done = add_edge_if_possible(rows.row(open), R, i))) break;
         }
     }
-    return rc.write_back();
+    return rows.write_back();
 }
 
 struct DevArr {
