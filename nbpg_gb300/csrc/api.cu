@@ -1,4 +1,7 @@
 // C ABI: index handles, data upload/download, error reporting.
+#include <sys/mman.h>
+#include <unistd.h>
+
 #include <cstring>
 #include <map>
 #include <mutex>
@@ -133,6 +136,15 @@ extern "C" nbpg_status nbpg_index_set_graph(nbpg_index *idx, const uint32_t *row
     return NBPG_OK;
 }
 
+// Has the pages of a host buffer made, without a change to what is in them.  A range that is no writable host memory is
+// left to the copy to judge.
+static void populate_pages(void *p, size_t bytes)
+{
+    constexpr int kPopulateWrite = 23;  // MADV_POPULATE_WRITE (Linux 5.14)
+    const uintptr_t page = uintptr_t(sysconf(_SC_PAGESIZE)), a = reinterpret_cast<uintptr_t>(p) / page * page;
+    madvise(reinterpret_cast<void *>(a), reinterpret_cast<uintptr_t>(p) + bytes - a, kPopulateWrite);
+}
+
 extern "C" nbpg_status nbpg_index_get_graph(const nbpg_index *cidx, uint32_t *rows, uint64_t first, uint64_t count)
 {
     auto *idx = const_cast<nbpg_index *>(cidx);
@@ -143,9 +155,8 @@ extern "C" nbpg_status nbpg_index_get_graph(const nbpg_index *cidx, uint32_t *ro
     NBPG_CUDA_TRY(cudaSetDevice(idx->desc.device));
     const uint32_t R = idx->desc.max_degree;
     // Pages of a fresh buffer that the copy is the first to touch are faulted in from the device, one at a
-    // time: 22 ms for the 26 MB of 100k rows, 0.5 ms once they are there.  The host touches them first.
-    const size_t bytes = size_t(count) * (R + 1) * 4;
-    for (size_t b = 0; b < bytes; b += 4096) *reinterpret_cast<volatile uint32_t *>(reinterpret_cast<uint8_t *>(rows) + b) = 0;
+    // time: 22 ms for the 26 MB of 100k rows, 0.5 ms once they are there.  So the kernel makes them first.
+    populate_pages(rows, size_t(count) * (R + 1) * 4);
     NBPG_CUDA_TRY(cudaMemcpy2DAsync(rows, (R + 1) * 4, idx->d_graph + first * idx->gstride, idx->gstride * 4,
                                     (R + 1) * 4, count, cudaMemcpyDeviceToHost, idx->stream));
     NBPG_CUDA_TRY(cudaStreamSynchronize(idx->stream));

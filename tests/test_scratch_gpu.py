@@ -128,3 +128,21 @@ for limit in (peak - 1, peak - room // 2, peak - room):
 assert build(peak // 3) is None
 assert build(1 << 40)[1] == want and shim.shim_overrun() == 0
 """)
+
+
+def test_get_graph_leaves_the_destination_to_the_copy(shim):
+    """A destination that the host cannot write is answered by the copy's status, and the process lives on."""
+    shim("""
+g = np.zeros((300, 9), np.uint32)
+g[:, 0], g[:, 1:4] = 3, r.integers(0, 300, (300, 3))
+idx = Index(r.integers(0, 256, (300, 16)).astype(np.uint8), "u8", "l2", max_degree=8, graph=g)
+other = Index(r.integers(0, 256, (4000, 16)).astype(np.uint8), "u8", "l2", max_degree=8)
+device = other.device_info()[2]
+status = _lib.lib().nbpg_index_get_graph(idx._h, C.cast(C.c_void_p(device), C.POINTER(C.c_uint32)), 0, 300)
+assert status in (0, 3), status
+live = np.arange(8)[None, :] < g[:, :1]
+got = idx.get_graph()
+assert np.array_equal(got[:, 0], g[:, 0]) and np.array_equal(got[:, 1:][live], g[:, 1:][live])
+idx.close()
+other.close()
+""")
