@@ -88,6 +88,7 @@ struct ReleaseOnExit {
 // Launches that may overlap on the device need separate scratch.
 struct SearchScratch {
     DevBuf queue, sp, ghash, gvis;
+    size_t refused = SIZE_MAX;        // smallest ghash + gvis that could not be had
     const uint32_t *order = nullptr;  // optional processing order of the next launch (device)
     std::vector<uint32_t> sp_host;  // start points currently in `sp`
     void release()

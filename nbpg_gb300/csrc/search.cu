@@ -412,12 +412,33 @@ nbpg_status search_device_impl(nbpg_index *idx, SearchScratch &sc, const void *d
     // so that one memset clears the counters: one query 87.5 -> 86.3 us); start points
     if ((s = sc.queue.ensure((size_t(nq) + 5) * sizeof(uint32_t))) != NBPG_OK) return s;
     if ((s = sc.sp.ensure(256 * sizeof(uint32_t))) != NBPG_OK) return s;
-    size_t nslots = std::max<size_t>(main.ghash || main.gvis ? size_t(main.grid) * main.warps : 0,
-                                     rerun.ghash || rerun.gvis ? size_t(rerun.grid) * rerun.warps : 0);
-    uint32_t hslots = std::max(main.ghash ? main.S : 0u, rerun.ghash ? rerun.S : 0u);
-    uint32_t vcap = std::max(main.gvis ? main.Vcap : 0u, rerun.gvis ? rerun.Vcap : 0u);
-    if (hslots && (s = sc.ghash.ensure(nslots * hslots * sizeof(uint32_t))) != NBPG_OK) return s;
-    if (vcap && (s = sc.gvis.ensure(nslots * vcap * sizeof(uint64_t))) != NBPG_OK) return s;
+    const uint32_t hslots = std::max(main.ghash ? main.S : 0u, rerun.ghash ? rerun.S : 0u);
+    const uint32_t vcap = std::max(main.gvis ? main.Vcap : 0u, rerun.gvis ? rerun.Vcap : 0u);
+    // A filter and a visited list per warp of the persistent grids; where that does not fit, fewer CTAs.  What was
+    // refused is remembered, so that a call that repeats another (the one that captures it) keeps its buffers.
+    while (true) {
+        const bool main_global = main.ghash || main.gvis, rerun_global = rerun.ghash || rerun.gvis;
+        const size_t nslots = std::max<size_t>(main_global ? size_t(main.grid) * main.warps : 0,
+                                               rerun_global ? size_t(rerun.grid) * rerun.warps : 0);
+        const size_t hash_bytes = nslots * hslots * sizeof(uint32_t), vis_bytes = nslots * vcap * sizeof(uint64_t);
+        if (hash_bytes + vis_bytes < sc.refused) {
+            s = hash_bytes ? sc.ghash.ensure(hash_bytes) : NBPG_OK;
+            if (s == NBPG_OK && vis_bytes) s = sc.gvis.ensure(vis_bytes);
+            if (s == NBPG_OK) break;
+            if (s != NBPG_ERR_OOM) return s;
+            cudaGetLastError();
+            sc.refused = hash_bytes + vis_bytes;
+            sc.ghash.release();
+            sc.gvis.release();
+        }
+        if ((!main_global || main.grid <= 1) && (!rerun_global || rerun.grid <= 1)) {
+            set_error("search scratch: out of memory");
+            sc.refused = SIZE_MAX;
+            return NBPG_ERR_OOM;
+        }
+        if (main_global) main.grid = std::max<uint32_t>(1, main.grid / 2);
+        if (rerun_global) rerun.grid = std::max<uint32_t>(1, rerun.grid / 2);
+    }
 
     uint32_t *q = sc.queue.as<uint32_t>(), *const taint = q + 4;
     NBPG_CUDA_TRY(cudaMemsetAsync(q, 0, 5 * sizeof(uint32_t), st));

@@ -146,3 +146,31 @@ assert np.array_equal(got[:, 0], g[:, 0]) and np.array_equal(got[:, 1:][live], g
 idx.close()
 other.close()
 """)
+
+
+@pytest.mark.parametrize("kernel", ["batched", "plain"])
+def test_search_runs_with_the_scratch_there_is(shim, kernel):
+    """Long beams keep a visited filter per warp in global memory: with less of it the grids are smaller and the results
+    the same."""
+    shim(f"kernel = {kernel!r}" + """
+base, q = synth.u8_mixture(4000, 600, dim=32, n_centres=24)
+idx = Index(base, "u8", "ip", max_degree=24)
+idx.build_vamana(L=32, VL=48, num_split=0, num_passes=1)
+for L in (300, 200):
+    qp = QueryParams(k=50, beamSize=L)
+    idx2 = Index(base, "u8", "ip", max_degree=24, graph=idx.get_graph())
+    want = idx2.search(q, qp, launch=LaunchConfig(kernel=kernel))
+    idx2.close()
+    for room in (100 << 20, 20 << 20, 4 << 20):  # (one CTA of 16 warps takes 2.6 MB at L = 300)
+        idx2 = Index(base, "u8", "ip", max_degree=24, graph=idx.get_graph())
+        shim.shim_limit(shim.shim_used() + room)
+        for _ in range(2):
+            got = idx2.search(q, qp, launch=LaunchConfig(kernel=kernel))
+            for a, b in zip((want.ids, want.dists, want.count, want.visited, want.cmps),
+                            (got.ids, got.dists, got.count, got.visited, got.cmps)):
+                assert np.array_equal(a, b), (L, room)
+        shim.shim_limit(1 << 40)
+        idx2.close()
+idx.close()
+assert shim.shim_overrun() == 0
+""")
