@@ -496,6 +496,7 @@ nbpg_status search_device_impl(nbpg_index *idx, SearchScratch &sc, const void *d
     m.g_hash_slots = main.ghash ? hslots : 0;
     m.g_vis = main.gvis ? sc.gvis.as<uint64_t>() : nullptr;
     m.g_vis_cap = main.gvis ? vcap : 0;
+    m.vis_most = rerun.Vcap;
     ops->launch(metric, pass, plain, plain ? nq : main.grid, main.warps, main.smem, m, st);
     NBPG_CUDA_TRY(cudaGetLastError());
 

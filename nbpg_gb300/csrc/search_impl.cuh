@@ -73,6 +73,7 @@ struct SearchArgs {
     uint32_t g_hash_slots;  // slots per warp slot in g_hash
     uint64_t *g_vis;        // global visited-list scratch (null = in shared memory)
     uint32_t g_vis_cap;
+    uint32_t vis_most;  // search_flag, inner product: the visited list that the re-run has room for
     uint32_t prefetch;  // unvisited entries whose adjacency rows are prefetched to L2
     uint32_t *err;      // set to 1 when a query's (L, k) is rejected
     // outputs for a re-rank with raw vectors (beam_search_rerank, beamSearch.h:183-247);

@@ -23,7 +23,8 @@ __device__ void search_query(const SearchArgs &a, uint32_t qi, uint8_t *slot, ui
     }
     if (L == 0 || k == 0 || k > L || L > a.lay.Lcap || nsp > L || k > a.k_stride ||
         (LIST && !a.g_vis && max_visited > a.lay.Vcap) || (!a.g_hash && S > a.lay.Scap) ||
-        (a.g_hash && S > a.g_hash_slots) || (LIST && a.g_vis && max_visited > a.g_vis_cap)) {
+        (a.g_hash && S > a.g_hash_slots) || (LIST && a.g_vis && max_visited > a.g_vis_cap) ||
+        (PASS == PASS_WIDE && MET == M_IP && max_visited > a.vis_most)) {
         // rejected (the reference aborts on k > L, beamSearch.h:268-273): empty row + error flag
         for (uint32_t j = lane; j < a.k_stride; j += 32) {
             a.out_ids[size_t(qi) * a.k_stride + j] = kNoId;

@@ -174,3 +174,29 @@ for L in (300, 200):
 idx.close()
 assert shim.shim_overrun() == 0
 """)
+
+
+@pytest.mark.parametrize("kernel", ["batched", "plain"])
+def test_beam_above_the_calls_is_refused_for_all_its_queries(gpu_lib, kernel):
+    """Inner product, a call of L = 19: the visited list of its exact re-run holds 160 entries, 8 per beam place.  A query
+    that asks for L = 21 is answered with an empty row whether or not it would have been run again."""
+    import numpy as np
+    import torch
+    from conftest import dataset
+    from nbpg_gb300.index import Index, LaunchConfig, QueryParams
+    base, q, g = dataset("i8", "ip")
+    idx = Index(base, "i8", "ip", max_degree=g.shape[1] - 1, graph=g)
+    rs, nq, k = idx.device_info()[1], len(q), 10
+    d = torch.zeros((nq, rs), dtype=torch.uint8, device="cuda")
+    d[:, :q.shape[1]] = torch.from_numpy(np.ascontiguousarray(q).view(np.uint8)).cuda()
+    Ls = torch.tensor([19, 20, 21] * nq, dtype=torch.int32, device="cuda")[:nq].contiguous()
+    ids = torch.full((nq, k), 7, dtype=torch.int32, device="cuda")
+    counts = torch.full((3, nq), 7, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    idx.search_device(d.data_ptr(), nq, QueryParams(k=k, beamSize=19), ids.data_ptr(), k, None, counts[0].data_ptr(),
+                      counts[1].data_ptr(), counts[2].data_ptr(), launch=LaunchConfig(kernel=kernel), d_Ls=Ls.data_ptr())
+    torch.cuda.synchronize()
+    refused = (Ls == 21).cpu().numpy()
+    got, found = ids.cpu().numpy(), counts[0].cpu().numpy()
+    assert (got[refused] == -1).all() and (found[refused] == 0).all()
+    assert (found[~refused] > 0).all() and (got[~refused, 0] >= 0).all()
