@@ -297,15 +297,16 @@ __device__ __forceinline__ uint32_t warp_upper_bound(const uint64_t *s, uint32_t
 
 // Probe and insert a chunk of neighbours (lanes with act) in the visited filter, in lane order.
 // Returns whether this lane's id was there.
-// GH: the filter is in global memory, where one round trip costs more than a match.
-// EITHER (LIST mode, where the kernel does not know): read after the match, by the lanes that need it; reading ahead
-// of the match took LIST mode 5% longer (8k inner-product queries on 1,000-byte rows, L = 16: 158 -> 170 us).
-template <bool GH, bool EITHER = false>
+// GH: the filter may be in global memory, where one round trip costs more than a match: it is read ahead of the match.
+// LATE: a match too, but the filter is read after it, by the lanes that need it.  One-warp blocks in LIST mode are 5%
+// faster so (8k inner-product queries on 1,000-byte rows, L = 16: 170 -> 160 us), the persistent ones 5 to 8% slower
+// (300 L2 queries on 2,048-byte rows at L = 33, most of them re-run: 153 -> 166 us).
+template <bool GH, bool LATE = false>
 __device__ __forceinline__ bool filter_probe(uint32_t *H, uint32_t smask, uint32_t nb, bool act)
 {
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t sl = act ? filter_slot(nb, smask) : kNoId;
-    if constexpr (EITHER) {
+    if constexpr (LATE) {
         const unsigned here = __match_any_sync(kFull, sl);
         const unsigned before = here & lanemask_lt();
         const uint32_t prev = __shfl_sync(kFull, nb, before ? 31 - __clz(before) : int(lane));
@@ -358,7 +359,7 @@ __device__ __forceinline__ bool filter_probe(uint32_t *H, uint32_t smask, uint32
 // whole warp on one query row.  slot: this warp's shared-memory slot; gslot: index of
 // its global scratch block; sp/nsp: start points; self: node excluded from expansion
 // (Points[a].same_as(p), beamSearch.h:79) or kNoId.  Leaves the frontier, visited list
-// and visited filter in place and describes them in the returned state.
+// and visited filter in place and describes them in the returned state.  LATE: see filter_probe.
 struct SearchState {
     uint64_t *fr0, *fr1, *vis;
     uint32_t *H;
@@ -371,7 +372,7 @@ struct SearchState {
     __device__ uint64_t *frontier() const { return b ? fr1 : fr0; }
 };
 
-template <int DT, int MET, bool LIST, int VPL>
+template <int DT, int MET, bool LIST, int VPL, bool LATE = false>
 __device__ SearchState search_core(const SearchArgs &a, const uint8_t *qrow_bytes, uint32_t L, uint32_t k,
                                    uint64_t max_visited, const uint32_t *sp, uint32_t nsp, uint8_t *slot,
                                    uint32_t gslot, int lane, uint32_t self)
@@ -495,7 +496,7 @@ __device__ SearchState search_core(const SearchArgs &a, const uint8_t *qrow_byte
             const uint32_t i = c * 32 + lane;
             const bool act = i < ne;
             const uint32_t nb = nbv[c];
-            const bool seen = filter_probe<false, LIST>(H, smask, nb, act);
+            const bool seen = filter_probe<LIST, LIST && LATE>(H, smask, nb, act);
             const bool keep = act && !seen && nb != self;
             const unsigned km = __ballot_sync(kFull, keep);
             if (keep) filt[nf + __popc(km & lanemask_lt())] = nb;

@@ -6,7 +6,7 @@
 namespace nbpg {
 
 // One query of a search request: argument checks, search_core, outputs.
-template <int DT, int MET, int PASS, int VPL, bool GH>
+template <int DT, int MET, int PASS, int VPL, bool GH, bool PLAIN = false>
 __device__ void search_query(const SearchArgs &a, uint32_t qi, uint8_t *slot, uint32_t gslot, int lane)
 {
     constexpr bool LIST = PASS == PASS_LIST;
@@ -51,7 +51,7 @@ __device__ void search_query(const SearchArgs &a, uint32_t qi, uint8_t *slot, ui
         frb = st.fr;
         fs = st.fs, cmps = st.cmps, adj = st.adj, nvis = st.nvis, taint = st.taint;
     } else {
-        const SearchState st = search_core<DT, MET, LIST, VPL>(a, qrow, L, k, max_visited, sp, nsp, slot, gslot, lane, kNoId);
+        const SearchState st = search_core<DT, MET, LIST, VPL, PLAIN>(a, qrow, L, k, max_visited, sp, nsp, slot, gslot, lane, kNoId);
         frb = st.frontier();
         vis = st.vis;
         fs = st.fs, cmps = st.cmps, adj = st.adj, nvis = st.nvis, taint = st.taint;
@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(32, 28) search_plain_kernel(SearchArgs a)
     const uint32_t total = a.only ? a.only[0] : a.nq;
     if (blockIdx.x >= total) return;
     const uint32_t qi = a.only ? a.only[1 + blockIdx.x] : (a.order ? a.order[blockIdx.x] : blockIdx.x);
-    search_query<DT, MET, PASS, VPL, false>(a, qi, smem, blockIdx.x, threadIdx.x);
+    search_query<DT, MET, PASS, VPL, false, true>(a, qi, smem, blockIdx.x, threadIdx.x);
 }
 
 }  // namespace nbpg
