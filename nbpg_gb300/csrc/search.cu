@@ -84,6 +84,17 @@ SlotLayout make_flag_layout(uint32_t Lmax, uint32_t R, uint32_t row_stride, bool
     return l;
 }
 
+// Calls that the flag kernels (search_flag.cuh) do not make faster, measured on 20k-row graphs of R = 32:
+//  - A few inner-product queries: their exact re-run is one launch more, 2 to 5 us on top of 28 to 50 (one query of 256
+//    bytes 28.5 us in LIST mode, 33.6 with both).  From 16 queries on the two are level, on the persistent kernel from 5,
+//    and there LIST mode is the slower one on long rows (4 queries of 2,048 bytes, L = 64: 86 us, 81 with both).
+//  - Rows above 512 bytes (four words a lane, 16 lanes a row) on the plain kernel, where few rows are in flight and the
+//    query's words are read again for each of them.  L2: 8k queries of 1,000 bytes at L = 64 335 us with search_core,
+//    433 with search_flag, at L = 150 1,084 and 1,299; also 4 to 9% where the caller asks for four words on short rows, and
+//    4 to 6% at 384 bytes.  Inner product: 8k queries of 2,048 bytes at L = 32 192 us in LIST mode, 204 with flags;
+//    at L = 100 337 and 309.
+static constexpr uint32_t kFewPlain = 12, kFewBatched = 4, kFewBeam = 128;
+
 // Thresholds for keeping per-query tables in shared memory.
 static constexpr uint32_t kHashSmemMax = 32768;  // bytes of visited filter per warp slot
 static constexpr uint32_t kVisSmemMax = 16384;   // bytes of visited list per warp slot
@@ -391,16 +402,19 @@ nbpg_status search_device_impl(nbpg_index *idx, SearchScratch &sc, const void *d
         return NBPG_OK;
     }
     const uint32_t vf = P->visited_factor ? P->visited_factor : 8;
-    // filtering mode needs the visited list itself; search_flag's inner-product frontier is 32 entries longer
-    // than its 1024 positions allow at the longest beams
-    const bool flag_first = !(emit && emit->visited) && !(metric == M_IP && P->L > 992);
+    // Filtering mode needs the visited list itself, and search_flag's inner-product frontier is 32 entries longer than its
+    // 1024 positions allow at the longest beams.
+    const bool long_rows = vecs > 32;
+    const bool few = P->L <= kFewBeam && (plain ? nq <= kFewPlain : nq <= kFewBatched && !long_rows);
+    const bool flag_first = !(emit && emit->visited) &&
+                            !(metric == M_IP && (P->L > 992 || few || (plain && long_rows && P->L < 64)));
     if (emit && emit->visited)
         NBPG_CHECK_ARG(k_stride >= (P->visited_factor ? P->visited_factor : 8) * P->L,
                        "k_stride must hold the visited list (visited_factor * L)");
 
     PassCfg main{}, rerun{};
-    // beams above 32 (the largest of the call) and inner product: search_flag
-    const int pass = !flag_first ? PASS_LIST : P->L > 32 || metric == M_IP ? PASS_WIDE : PASS_FLAG;
+    const bool wide = metric == M_IP || (P->L > 32 && !(plain && (vpl == 4 || lpr >= 16)));
+    const int pass = !flag_first ? PASS_LIST : wide ? PASS_WIDE : PASS_FLAG;
     nbpg_status s = plan_pass(idx, ops, metric, pass, plain, P->L, vf, P->warps_per_cta, main);
     if (s != NBPG_OK) return s;
     if (flag_first) {
@@ -510,7 +524,8 @@ nbpg_status search_device_impl(nbpg_index *idx, SearchScratch &sc, const void *d
         r.g_vis = rerun.gvis ? sc.gvis.as<uint64_t>() : nullptr;
         r.g_vis_cap = rerun.gvis ? vcap : 0;
         r.prefetch = 0;
-        ops->launch(metric, PASS_LIST, false, rerun.grid, rerun.warps, rerun.smem, r, st);
+        // (no more CTAs than queries; a few re-run queries spread over the SMs)
+        ops->launch(metric, PASS_LIST, false, std::min(rerun.grid, nq), rerun.warps, rerun.smem, r, st);
         NBPG_CUDA_TRY(cudaGetLastError());
     }
     return NBPG_OK;
