@@ -77,11 +77,21 @@ __device__ __forceinline__ uint32_t pca_col(uint32_t tx, int o)
     return o < 4 ? tx * 4 + o : 32 + tx * (OPT - 4) + (o - 4);
 }
 
+// What a column of staged matrix row i is XORed with: the transposing stores of a warp (32 rows of one column) go to 8
+// banks instead of one, and a thread's vector stays one vector (1,000 rows of 576 codes -> 128: 65 -> 53 us; 1M x 128 ->
+// 64: 673 -> 620).  48 columns are 16 banks apart from row to row, and gain less from it than the address costs (200k x
+// 128 -> 34: 123 us without, 131 with).
+template <int OPT>
+__device__ __forceinline__ uint32_t pca_swizzle(uint32_t i)
+{
+    return OPT == 6 ? 0 : 4 * (i & 7);
+}
+
 // One CTA: 32 * PPT points x 8 * OPT outputs; a thread owns PPT points x OPT outputs in registers
 // and walks the input elements in index order, so every output keeps the reference's summation order.
 // What bounds it: one multiply and one add per input element and output (two instructions, no FMA):
 // 16.4 G lane operations for 1M x 128 -> 64, 0.42 ms on 152 SMs x 128 lanes at 2 GHz, against 0.08 ms
-// of HBM traffic; it measures 0.67 ms (1.70 ms with one output x 8 points per thread, a whole d_in of
+// of HBM traffic; it measures 0.62 ms (1.70 ms with one output x 8 points per thread, a whole d_in of
 // both operands in shared memory and double-precision quantisation).  Hence a register tile (16 shared-memory values feed 64 multiply-adds) and
 // two-wide mul / add, which leave issue slots for the loads.  xs[i][p] is stored with its point
 // index XORed by 4 * ((i / 4) % 8): the transposing stores and the 16-byte reads are both free of
@@ -147,7 +157,7 @@ __global__ void __launch_bounds__(PCA_THREADS, 2) pca_kernel(const void *x, uint
         }
         for (uint32_t e = tid; e < O * PCA_KC; e += PCA_THREADS) {
             const uint32_t i = e % PCA_KC, j = e / PCA_KC;
-            ms[i * O + j] = i < kc && j0 + j < d_out ? __ldg(mat + size_t(j0 + j) * d_in + i0 + i) : 0.0f;
+            ms[i * O + (j ^ pca_swizzle<OPT>(i))] = i < kc && j0 + j < d_out ? __ldg(mat + size_t(j0 + j) * d_in + i0 + i) : 0.0f;
         }
         __syncthreads();
         for (uint32_t i = 0; i < kc; ++i) {
@@ -171,13 +181,13 @@ __global__ void __launch_bounds__(PCA_THREADS, 2) pca_kernel(const void *x, uint
             uint64_t mv[OPT / 2];
             const float *mr = ms + i * O;
             {
-                const ulonglong2 t = *reinterpret_cast<const ulonglong2 *>(mr + tx * 4);
+                const ulonglong2 t = *reinterpret_cast<const ulonglong2 *>(mr + ((tx * 4) ^ pca_swizzle<OPT>(i)));
                 mv[0] = t.x;
                 mv[1] = t.y;
             }
             if constexpr (OPT == 6) mv[2] = *reinterpret_cast<const uint64_t *>(mr + 32 + tx * 2);
             if constexpr (OPT == 8) {
-                const ulonglong2 t = *reinterpret_cast<const ulonglong2 *>(mr + 32 + tx * 4);
+                const ulonglong2 t = *reinterpret_cast<const ulonglong2 *>(mr + 32 + ((tx * 4) ^ pca_swizzle<OPT>(i)));
                 mv[2] = t.x;
                 mv[3] = t.y;
             }
@@ -306,8 +316,9 @@ static nbpg_status launch_pca(uint32_t in_dtype, const void *d_x, uint64_t n, ui
                               const float *d_bias, uint32_t d_out, uint32_t out_dtype, void *d_out_rows,
                               cudaStream_t st)
 {
-    // columns per CTA: 32 or 48 where they cover d_out (no columns computed for padding), else 64
-    const uint32_t opt = d_out <= 32 ? 4 : d_out <= 48 ? 6 : 8;
+    // columns per CTA: 32 or 48 where they cover d_out (no columns computed for padding), else 64; 48 for many points
+    // only (1,000 rows of 128 -> 34: 22.3 us with 48 columns, 21.1 with 64; 20,000: 33 and 35)
+    const uint32_t opt = d_out <= 32 ? 4 : d_out <= 48 && n >= 8192 ? 6 : 8;
     // 256-point tiles once they fill every SM's two CTAs (2 x 152 x 256 = 78k points), else 64-point ones
     const uint32_t ppt = n >= 80000 ? 8 : 2;
     const uint32_t pts = 32 * ppt, outs = 8 * opt;
