@@ -626,8 +626,10 @@ __global__ void __launch_bounds__(128) gt_replay_kernel(ReplayArgs a)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t q = blockIdx.x * 4 + warp, k = a.k;
     if (blockIdx.x == 0 && threadIdx.x == 0) *a.s.pool_next = 0;  // for the next stage
-    if (q >= a.s.nq || *a.s.err) return;
-    if (a.ovf && a.ovf[q]) return;  // (nothing was recorded either: its bound is below every distance)
+    if (q >= a.s.nq) return;
+    // read together; a query whose records were lost has recorded nothing more (its bound is below every distance)
+    const uint32_t err = *a.s.err, gone = a.ovf ? a.ovf[q] : 0u;
+    if (err | gone) return;
     uint64_t *buf = bufs[warp];
     CgList cg{};
     ExList ex{};
