@@ -299,7 +299,7 @@ nbpg_status nbpg_gt(uint32_t dtype, uint32_t metric, uint32_t dims, const void *
                     float *out_dists, int32_t device);
 
 /* Distance engine for nbpg_gt_with_engine: AUTO picks the tensor engine where it applies (row
- * length up to 640 codes after 4-bit expansion, k <= 128) and DP4A otherwise; TENSOR takes rows
+ * length up to 576 codes after 4-bit expansion, k <= 128) and DP4A otherwise; TENSOR takes rows
  * of up to 128 codes and k <= 100 and returns NBPG_ERR_UNSUPPORTED past that.  Results are
  * identical across engines. */
 typedef enum nbpg_gt_engine { NBPG_GT_AUTO = 0, NBPG_GT_DP4A = 1, NBPG_GT_TENSOR = 2 } nbpg_gt_engine;

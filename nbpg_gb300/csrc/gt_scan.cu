@@ -19,7 +19,7 @@
 //
 // Exactness: u8 codes are centred by 128 (L2 does not change; the inner product is corrected with
 // the rows' code sums), so that all codes are below 2^8 in magnitude, exact in bf16, and a dot
-// product of up to 640 of them is an integer below 2^24, exact in the fp32 accumulator.  The chunk
+// product of up to 640 of them (the shared memory takes 576) is an integer below 2^24, exact in the fp32 accumulator.  The chunk
 // test runs in fp32, widened by `slack` where its values may pass 2^24; what it flags is decided on
 // the int32 distance, converted to float as the reference does (point.h:35-135).
 #include <cuda_bf16.h>
@@ -113,9 +113,7 @@ __device__ __forceinline__ void tc_ld32_wait(uint32_t (&v)[32])
 }
 
 // One lane of a converged warp.  The producer and the MMA warp run their loops with all lanes and
-// issue through this: the operands of TMA and tcgen05 instructions live in uniform registers, and
-// under a plain lane test the compiler serves each of them through a loop over the active lanes (193
-// cycles per 64-cycle MMA).
+// issue through this: 10k x 1M x 128, k = 100 took 4.90 ms with it and 5.80 with a test of the lane.
 __device__ __forceinline__ bool elect_one()
 {
     uint32_t one;
@@ -841,8 +839,8 @@ static uint32_t scan_ring(uint32_t katoms, size_t smem_optin)
     return 0;
 }
 
-// Whether the staged tensor scan applies: rows of up to 640 codes (query tile and ring in shared
-// memory, exact dot products), k up to 128 (the replay's registers).
+// Whether the staged tensor scan applies: rows of up to 576 codes (query tile and ring in shared
+// memory; dot products are exact up to 640), k up to 128 (the replay's registers).
 bool gt_scan_supported(uint32_t dtype, uint32_t dims, uint32_t k, size_t smem_optin)
 {
     if (dtype > NBPG_I4 || dims == 0 || dims > SC_MAX_ELEMS || k == 0 || k > SC_MAX_K) return false;

@@ -423,7 +423,7 @@ nbpg_status search_device_impl(nbpg_index *idx, SearchScratch &sc, const void *d
     }
 
     // scratch: [0] queue main, [1] queue rerun, [2] error word, [4] queries to re-run and their list (one buffer,
-    // so that one memset clears the counters: one query 87.5 -> 86.3 us); start points
+    // so that one memset clears the counters); start points
     if ((s = sc.queue.ensure((size_t(nq) + 5) * sizeof(uint32_t))) != NBPG_OK) return s;
     if ((s = sc.sp.ensure(256 * sizeof(uint32_t))) != NBPG_OK) return s;
     const uint32_t hslots = std::max(main.ghash ? main.S : 0u, rerun.ghash ? rerun.S : 0u);
